@@ -276,6 +276,65 @@ __global__ void depth_level(const uint32_t* frontier, uint32_t K, const uint32_t
     }
 }
 
+// One four-wide node for wide_walk.cu, 16 words: corner and step of the byte
+// planes per axis, lower planes (a byte per child) per axis, upper planes,
+// then per child the inner node's index or the leaf's reference. Inner
+// children come first, so that child k of them is node (word 12) + k. The
+// low four bits of the x step say which children are inner nodes, those of
+// the y step which are leaves. Boxes are rounded outwards by at least 1/64
+// of a step (more than the walk's arithmetic loses on the bytes).
+__global__ void wide_nodes(const uint4* bvh4, uint32_t n4, uint32_t* out) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n4) return;
+    const uint4* nd = bvh4 + (size_t)i * 8;
+    const uint4 rf = nd[6];
+    const uint32_t ref[4] = {rf.x, rf.y, rf.z, rf.w};
+    int from[4], kids = 0, inner = 0;  // child j of the new node is child from[j]
+    for (int pass = 0; pass < 2; pass++)
+        for (int k = 0; k < 4; k++)
+            if (ref[k] != NONE && ((ref[k] & LEAF) != 0u) == (pass == 1)) {
+                from[kids++] = k;
+                inner += pass == 0;
+            }
+    uint32_t w[16];
+    for (int ax = 0; ax < 3; ax++) {
+        const uint4 l4 = nd[ax], h4 = nd[3 + ax];
+        const float lo[4] = {__uint_as_float(l4.x), __uint_as_float(l4.y), __uint_as_float(l4.z), __uint_as_float(l4.w)};
+        const float hi[4] = {__uint_as_float(h4.x), __uint_as_float(h4.y), __uint_as_float(h4.z), __uint_as_float(h4.w)};
+        float mn = 3.0e38f, mx = -3.0e38f;
+        for (int j = 0; j < kids; j++) {
+            mn = fminf(mn, lo[from[j]]);
+            mx = fmaxf(mx, hi[from[j]]);
+        }
+        float step = fmaxf((mx - mn) * (1.0f / 253.0f), fmaxf(fmaxf(fabsf(mn), fabsf(mx)) * 1.0e-7f, 1.0e-30f));
+        const uint32_t mask = ax == 0 ? (1u << inner) - 1u : (ax == 1 ? (1u << kids) - (1u << inner) : 0u);
+        step = __uint_as_float((__float_as_uint(step) & ~15u) | mask);
+        const float corner = mn - step * 0.5f;
+        uint32_t ql = 0, qh = 0;
+        for (int j = 0; j < kids; j++) {
+            const uint32_t a = (uint32_t)fminf(fmaxf(floorf((lo[from[j]] - corner) / step - 0.015625f), 0.0f), 255.0f);
+            const uint32_t b = (uint32_t)fminf(fmaxf(ceilf((hi[from[j]] - corner) / step + 0.015625f), 0.0f), 255.0f);
+            ql |= a << (8 * j);
+            qh |= b << (8 * j);
+        }
+        w[ax] = __float_as_uint(corner);
+        w[3 + ax] = __float_as_uint(step);
+        w[6 + ax] = ql;
+        w[9 + ax] = qh;
+    }
+    for (int j = 0; j < 4; j++) w[12 + j] = j < kids ? ref[from[j]] : 0u;
+    uint4* o = reinterpret_cast<uint4*>(out) + (size_t)i * 4;
+    for (int k = 0; k < 4; k++) o[k] = make_uint4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+}
+
+__global__ void leaf_map(const uint32_t* w, uint32_t nodes, uint32_t* map, uint32_t slots) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nodes) return;
+    const uint32_t first = w[(size_t)i * 8 + 3], count = w[(size_t)i * 8 + 7];
+    if (count > slots || first > slots - count) return;
+    for (uint32_t k = 0; k < count; k++) map[first + k] = i;
+}
+
 unsigned blocks(uint32_t n, unsigned t) { return (n + t - 1) / t; }
 
 }  // namespace bvh4b
@@ -295,7 +354,7 @@ unsigned blocks(uint32_t n, unsigned t) { return (n + t - 1) / t; }
     } while (0)
 
 Collapse collapse4_device(const uint32_t* w, uint32_t nodes, cudaStream_t st, uint32_t** out, size_t* out_cap, uint32_t* n4,
-                          uint32_t* root_ref, uint32_t* need, std::string* err) {
+                          uint32_t* root_ref, uint32_t* need, std::string* err, size_t more_per_node, size_t more) {
     using namespace bvh4b;
     *n4 = 0;
     *need = 1;
@@ -375,12 +434,15 @@ Collapse collapse4_device(const uint32_t* w, uint32_t nodes, cudaStream_t st, ui
         sizes<<<blocks(e - s, 128), 128, 0, st>>>(items, s, e);
     }
     CK4(cudaGetLastError());
-    if (!*out || *out_cap < (size_t)*n4 * 128) {  // the caller's buffer, when it is large enough
-        if (*out) cudaFree(*out);
-        *out = nullptr;
-        *out_cap = 0;
-        CK4(cudaMalloc((void**)out, (size_t)*n4 * 128));
-        *out_cap = (size_t)*n4 * 128;
+    {
+        const size_t bytes = (size_t)*n4 * (128 + more_per_node) + more + 4;
+        if (!*out || *out_cap < bytes) {  // the caller's buffer, when it is large enough
+            if (*out) cudaFree(*out);
+            *out = nullptr;
+            *out_cap = 0;
+            CK4(cudaMalloc((void**)out, bytes));
+            *out_cap = bytes;
+        }
     }
     CK4(cudaMemsetAsync(ctr, 0, 4, st));
     for (size_t l = 0; l + 1 < level_start.size(); l++) {
@@ -459,5 +521,18 @@ done:
 }
 #undef CKD
 #undef CK4
+
+cudaError_t launch_wide_nodes(const uint4* bvh4, uint32_t n4, uint32_t* out, cudaStream_t st) {
+    if (n4 == 0) return cudaSuccess;
+    bvh4b::wide_nodes<<<bvh4b::blocks(n4, 128), 128, 0, st>>>(bvh4, n4, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_leaf_map(const uint32_t* words, uint32_t nodes, uint32_t* map, uint32_t slots, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(map, 0, (size_t)slots * 4, st);
+    if (e != cudaSuccess || nodes == 0) return e;
+    bvh4b::leaf_map<<<bvh4b::blocks(nodes, 256), 256, 0, st>>>(words, nodes, map, slots);
+    return cudaGetLastError();
+}
 
 }  // namespace oxd

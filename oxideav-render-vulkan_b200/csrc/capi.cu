@@ -115,7 +115,8 @@ struct oxpt_ctx {
     uint32_t check_every = 4;
     uint32_t shade_variant = 1, trace_variant = 4, nee_variant = 3, stack = 0;
     uint32_t bvh_depth = 0;
-    // four-wide any-hit tree (host/bvh4.cpp), built on upload when exact
+    // four-wide tree (host/bvh4.cpp), built on upload when exact; behind its
+    // nodes what wide_walk.cu reads (wide_part below)
     float4* bvh4 = nullptr;
     bool bvh4_built = false;
     uint32_t bvh4_nodes = 0, bvh4_root = 0xffffffffu, bvh4_need = 0;
@@ -202,6 +203,12 @@ oxpt_status realloc_dev(oxpt_ctx* c, T** p, size_t bytes, const char* what) {
     return OXPT_OK;
 }
 
+// The four-wide tree's buffer: 128 bytes a node, then 64 bytes a node
+// (Scene::wide), then a word per slot (Scene::leaf_of).
+constexpr size_t WIDE_NODE_BYTES = 64;
+size_t tree_bytes(uint32_t n4, size_t slots) { return (size_t)n4 * (128 + WIDE_NODE_BYTES) + (slots + 1) * 4; }
+uint32_t* wide_part(float4* bvh4, uint32_t n4) { return reinterpret_cast<uint32_t*>(bvh4 + (size_t)n4 * 8); }
+
 // The four-wide tree answers any-hit queries exactly when it was built from
 // the whole tree the params name and the binary walk it replaces never
 // overflows its 64-entry stack (at most 64 levels).
@@ -247,6 +254,8 @@ oxd::Scene scene_view(const oxpt_ctx* c) {
     s.P = c->params;
     if (bvh4_usable(c)) {
         s.bvh4 = c->bvh4;
+        s.wide = wide_part(c->bvh4, c->bvh4_nodes);
+        s.leaf_of = s.wide + (size_t)c->bvh4_nodes * 16;
         s.bvh4_root = c->bvh4_root;
         s.bvh4_nodes = c->bvh4_nodes;
         s.bvh4_ok = 1u;
@@ -461,6 +470,7 @@ oxpt_status run_wave(oxpt_ctx* c, const oxd::TraceArgs& ta, bool count, const ox
     wa.l2_share = c->l2_setaside / 2;  // two trees: binary for closest hits, four-wide for shadows
     wa.l2_max_window = c->l2_max_window;
     wa.closest4 = (c->closest_walk && c->trace_variant >= 3 && bvh4_usable(c)) ? 1u : 0u;
+    wa.wide = bvh4_usable(c) ? 1u : 0u;
     // Stack depth: 32 entries are exact when the BVH has at most 32 levels.
     int sd = c->stack ? (int)c->stack : (c->bvh_depth <= 32 ? 32 : 64);
     bool four = c->shadow_walk == 0 && bvh4_usable(c);
@@ -509,13 +519,14 @@ int enqueue_iteration(oxpt_ctx* c, const oxd::WaveArgs& wa, const oxd::WaveArgs&
     } else {
         run(2, [&] { return oxd::launch_wave_logic(wa, count, (int)c->shade_variant, st); });
     }
+    const int sde = (wa.closest4 || (wa.wide && !count && c->trace_variant >= 3)) ? sd4 : sd;
     if (wa.ray_order & 1u) {
         run(10, [&] { return oxd::launch_order_ext(wa, c->sms, st); });
         oxd::WaveArgs wo = wa;
         wo.q.ext = wa.q.ext_sorted;
-        run(3, [&] { return oxd::launch_wave_extend(wo, count, (int)c->trace_variant, wa.closest4 ? sd4 : sd, c->sms, st); });
+        run(3, [&] { return oxd::launch_wave_extend(wo, count, (int)c->trace_variant, sde, c->sms, st); });
     } else {
-        run(3, [&] { return oxd::launch_wave_extend(wa, count, (int)c->trace_variant, wa.closest4 ? sd4 : sd, c->sms, st); });
+        run(3, [&] { return oxd::launch_wave_extend(wa, count, (int)c->trace_variant, sde, c->sms, st); });
     }
     if ((wa.ray_order & 2u) && c->trace_variant >= 3)
         run(10, [&] { return oxd::launch_order_shadow(wa, c->sms, st); });
@@ -733,14 +744,15 @@ oxpt_status oxpt_device_summary(const oxpt_ctx* c, char* buf, size_t len) {
 static oxpt_status install_bvh4(oxpt_ctx* c, bool ok, const std::vector<uint32_t>& words, uint32_t root) {
     c->bvh4_built = false;
     if (!ok) return OXPT_OK;  // the binary walk serves every ray
-    oxpt_status s = reserve_dev(c, &c->bvh4, &c->bvh4_cap, words.size() * 4, "four-wide tree");
+    const uint32_t nodes = (uint32_t)(words.size() / oxpt::BVH4_NODE_WORDS);
+    oxpt_status s = reserve_dev(c, &c->bvh4, &c->bvh4_cap, tree_bytes(nodes, c->slot_count), "four-wide tree");
     if (s) return s;
     if (!words.empty()) {
         CK(c, cudaMemcpyAsync(c->bvh4, words.data(), words.size() * 4, cudaMemcpyHostToDevice, c->stream),
            "four-wide tree upload");
         CK(c, cudaStreamSynchronize(c->stream), "four-wide tree upload");
     }
-    c->bvh4_nodes = (uint32_t)(words.size() / oxpt::BVH4_NODE_WORDS);
+    c->bvh4_nodes = nodes;
     c->bvh4_root = root;
     c->bvh4_need = oxpt::bvh4_stack_need(words, root);
     c->bvh4_built = true;
@@ -754,6 +766,22 @@ static oxpt_status upload_bvh4(oxpt_ctx* c, const uint32_t* node_words, uint32_t
     return install_bvh4(c, ok, words, root);
 }
 
+// Fills the part of the four-wide tree's buffer that wide_walk.cu reads, from
+// the scene's two trees, on `st`.
+static oxpt_status build_wide(oxpt_ctx* c, const float4* geom, uint32_t nodes, size_t slots, float4** bvh4,
+                              size_t* cap, uint32_t n4, cudaStream_t st) {
+    if (*cap < tree_bytes(n4, slots)) {  // a root that is a leaf: no nodes were stored
+        oxpt_status s = realloc_dev(c, bvh4, tree_bytes(n4, slots), "four-wide tree");
+        *cap = s ? 0 : tree_bytes(n4, slots);
+        if (s) return s;
+    }
+    uint32_t* out = wide_part(*bvh4, n4);
+    CK(c, oxd::launch_wide_nodes(reinterpret_cast<const uint4*>(*bvh4), n4, out, st), "wide nodes");
+    CK(c, oxd::launch_leaf_map(reinterpret_cast<const uint32_t*>(geom), nodes, out + (size_t)n4 * 16, (uint32_t)slots,
+                               st), "leaf map");
+    return OXPT_OK;
+}
+
 // The four-wide tree of the scene now in c->geom, collapsed on the device
 // (the host collapse's words); a tree too wide or deep for the device pass
 // is read back and collapsed on the host.
@@ -763,18 +791,25 @@ static oxpt_status device_bvh4(oxpt_ctx* c) {
     uint32_t n4 = 0, root = 0xffffffffu, need = 1;
     std::string e;
     const uint32_t* words = reinterpret_cast<const uint32_t*>(c->geom);
-    oxd::Collapse r = oxd::collapse4_device(words, c->node_count, c->stream, &out, &c->bvh4_cap, &n4, &root, &need, &e);
+    oxd::Collapse r = oxd::collapse4_device(words, c->node_count, c->stream, &out, &c->bvh4_cap, &n4, &root, &need, &e,
+                                            WIDE_NODE_BYTES, c->slot_count * 4);
     c->bvh4 = reinterpret_cast<float4*>(out);
     if (r == oxd::Collapse::FAILED) return fail(c, OXPT_E_CUDA, e);
     if (r == oxd::Collapse::REFUSED) return OXPT_OK;  // the binary walk serves every ray
     if (r == oxd::Collapse::UNSUPPORTED) {
         std::vector<uint32_t> host((size_t)c->node_count * 8);
         CK(c, cudaMemcpy(host.data(), c->geom, host.size() * 4, cudaMemcpyDeviceToHost), "node readback");
-        return upload_bvh4(c, host.data(), c->node_count);
+        if (oxpt_status s = upload_bvh4(c, host.data(), c->node_count)) return s;
+        if (!c->bvh4_built) return OXPT_OK;
+    } else {
+        c->bvh4_nodes = n4;
+        c->bvh4_root = root;
+        c->bvh4_need = need;
     }
-    c->bvh4_nodes = n4;
-    c->bvh4_root = root;
-    c->bvh4_need = need;
+    c->bvh4_built = false;
+    if (oxpt_status s = build_wide(c, c->geom, c->node_count, c->slot_count, &c->bvh4, &c->bvh4_cap, c->bvh4_nodes,
+                                   c->stream))
+        return s;
     c->bvh4_built = true;
     return OXPT_OK;
 }
@@ -874,13 +909,15 @@ oxpt_status oxpt_stage_scene(oxpt_ctx* c, const oxpt_scene_desc* d, const uint32
     b.bvh4_built = false;
     uint32_t* out = reinterpret_cast<uint32_t*>(b.bvh4);
     uint32_t n4 = 0, root = 0xffffffffu, need = 1;
-    oxd::Collapse r = oxd::collapse4_device(words, d->node_count, c->upload, &out, &b.bvh4_cap, &n4, &root, &need, &e);
+    oxd::Collapse r = oxd::collapse4_device(words, d->node_count, c->upload, &out, &b.bvh4_cap, &n4, &root, &need, &e,
+                                            WIDE_NODE_BYTES, b.slot_count * 4);
     b.bvh4 = reinterpret_cast<float4*>(out);
     if (r == oxd::Collapse::FAILED) return fail(c, OXPT_E_CUDA, e);
     if (r == oxd::Collapse::BUILT) {
         b.bvh4_nodes = n4;
         b.bvh4_root = root;
         b.bvh4_need = need;
+        if ((s = build_wide(c, b.geom, b.node_count, b.slot_count, &b.bvh4, &b.bvh4_cap, n4, c->upload))) return s;
         b.bvh4_built = true;
     }
     // REFUSED / UNSUPPORTED: the binary walk serves every ray of this scene.
@@ -1488,7 +1525,7 @@ oxpt_status oxpt_ctx_memory(const oxpt_ctx* c, uint64_t out[4]) {
     uint64_t scene = 0;
     if (!c->borrowed_scene && c->has_scene) {
         scene = (uint64_t)c->geom_vec4 * 16 + (uint64_t)c->slot_count * 192 +
-                (uint64_t)c->side * c->side * c->layers * 8 + (uint64_t)c->bvh4_nodes * 128;
+                (uint64_t)c->side * c->side * c->layers * 8 + (c->bvh4_built ? tree_bytes(c->bvh4_nodes, c->slot_count) : 0);
     }
     scene += c->back.geom_cap + c->back.attrs_cap + c->back.atlas_cap + c->back.bvh4_cap;
     out[0] = scene;
@@ -1663,7 +1700,7 @@ oxpt_status batch_graph_run(oxpt_ctx* e, const std::vector<oxd::WaveArgs>& args,
         // node words (one-scene batches), the walk's storage split and tree.
         const oxd::WaveArgs& a0 = args[0];
         key.insert(key.end(), {(uint64_t)(uintptr_t)a0.s.geom, a0.s.geom_vec4, a0.s.P.env[3], a0.one_scene,
-                               a0.closest4, a0.walk_lim, a0.walk_stage, (uint64_t)(uintptr_t)a0.st.vis,
+                               a0.closest4, a0.wide, a0.walk_lim, a0.walk_stage, (uint64_t)(uintptr_t)a0.st.vis,
                                a0.shadow_post, a0.ray_order, a0.l2_share, a0.l2_max_window});
     }
     for (size_t k = 0; k < rounds.size(); k++) {
@@ -1859,7 +1896,7 @@ oxpt_status oxpt_refine_batch(oxpt_ctx* e, const oxpt_batch_frame* fr, uint32_t 
             J = std::max(J, c->params.cfg[2] + 1u);
             max_bounces = std::max(max_bounces, c->params.dims[3]);
             if (c->bvh_depth > 32) sd = 64;
-            if ((e->shadow_walk == 0 || e->closest_walk) && bvh4_usable(c) && c->bvh4_need > 32) sd = 64;
+            if (bvh4_usable(c) && c->bvh4_need > 32) sd = 64;
         }
     // Records go through pinned staging: the host waits only until the
     // previous batch's records were copied, not for that batch to finish.
@@ -1893,9 +1930,10 @@ oxpt_status oxpt_refine_batch(oxpt_ctx* e, const oxpt_batch_frame* fr, uint32_t 
         wa.total = total;
         args.push_back(wa);
     }
-    bool closest4 = e->closest_walk && e->trace_variant >= 3;
+    bool wide = true;  // every frame's scene has its four-wide tree
     for (uint32_t k = 0; k < n; k++)
-        if (fr[k].count && fr[k].rows && !bvh4_usable(fr[k].ctx)) closest4 = false;
+        if (fr[k].count && fr[k].rows && !bvh4_usable(fr[k].ctx)) wide = false;
+    const bool closest4 = e->closest_walk && e->trace_variant >= 3 && wide;
     oxd::WaveArgs base{};
     {
         // One scene for every frame (a single tracer's refine, or views of
@@ -1934,6 +1972,7 @@ oxpt_status oxpt_refine_batch(oxpt_ctx* e, const oxpt_batch_frame* fr, uint32_t 
         wa.l2_share = e->l2_setaside / 2;
         wa.l2_max_window = e->l2_max_window;
         wa.closest4 = closest4 ? 1u : 0u;
+        wa.wide = wide ? 1u : 0u;
         wa.total = total;
         wa.out = e->out;
         wa.counters = nullptr;
@@ -1942,9 +1981,7 @@ oxpt_status oxpt_refine_batch(oxpt_ctx* e, const oxpt_batch_frame* fr, uint32_t 
         wa.nframes = (uint32_t)rounds[k].size();
         off += rounds[k].size();
     }
-    bool four = e->shadow_walk == 0;
-    for (uint32_t k = 0; k < n; k++)
-        if (fr[k].count && fr[k].rows && !bvh4_usable(fr[k].ctx)) four = false;
+    const bool four = e->shadow_walk == 0 && wide;
     auto enqueue_reduces = [&](size_t k, cudaStream_t st) -> cudaError_t {
         for (const oxpt::BatchPiece& pc : rounds[k]) {
             oxpt_ctx* c = fr[pc.frame].ctx;

@@ -112,6 +112,10 @@ struct Scene {
     // bvh4_ok: 1 when it answers this scene's any-hit queries exactly.
     const float4* bvh4 = nullptr;
     uint32_t bvh4_root = 0xffffffffu, bvh4_nodes = 0u, bvh4_ok = 0u, pad_ = 0u;
+    // Set with bvh4: the same nodes with 8-bit child boxes (64 bytes each,
+    // wide_nodes in bvh4_build.cu), and the binary leaf node of every slot.
+    const uint32_t* wide = nullptr;
+    const uint32_t* leaf_of = nullptr;
 };
 
 __device__ __forceinline__ uint32_t tw(const Scene& s, uint32_t i) {

@@ -28,16 +28,24 @@ bool build_on_device(const float* pos, uint32_t n, cudaStream_t st, uint32_t** w
 // device memory (bvh4_build.cu): the host collapse's words (host/bvh4.cpp),
 // node for node. BUILT: *out holds n4 x 32 words (the caller's buffer of
 // *out_cap bytes when large enough, else a new cudaMalloc that replaces
-// it; untouched when the root is a leaf), *root_ref and *need are set. REFUSED: the host collapse
+// it; untouched when the root is a leaf; with room for more_per_node bytes a
+// node and `more` behind the nodes), *root_ref and *need are set. REFUSED: the host collapse
 // refuses the tree too (keep the binary walk). UNSUPPORTED: deeper than
 // 64 four-wide levels (collapse on the host). FAILED: a CUDA error.
 enum class Collapse { BUILT, REFUSED, UNSUPPORTED, FAILED };
 Collapse collapse4_device(const uint32_t* words, uint32_t nodes, cudaStream_t st, uint32_t** out, size_t* out_cap,
                           uint32_t* n4,
-                          uint32_t* root_ref, uint32_t* need, std::string* err);
+                          uint32_t* root_ref, uint32_t* need, std::string* err, size_t more_per_node = 0,
+                          size_t more = 0);
 // Levels of the binary tree (65 when deeper than 64 or malformed), as the
 // host's depth walk counts them.
 bool binary_depth_device(const uint32_t* words, uint32_t nodes, cudaStream_t st, uint32_t* depth, std::string* err);
+// The four-wide nodes with 8-bit child boxes, 16 words each: lower corner and
+// step per axis, a byte per child and plane, the child references.
+cudaError_t launch_wide_nodes(const uint4* bvh4, uint32_t n4, uint32_t* out, cudaStream_t st);
+// map[slot] = the binary leaf node that holds the slot, for every slot below
+// `slots` (0 for a slot in no leaf).
+cudaError_t launch_leaf_map(const uint32_t* words, uint32_t nodes, uint32_t* map, uint32_t slots, cudaStream_t st);
 
 namespace prep {
 

@@ -328,7 +328,9 @@ void* kernel_c(bool ext, bool four, bool post, int v, int sd) {
     if (ext && four) return sd <= 32 ? ext4_fn<C, 32, B>(v) : ext4_fn<C, 64, B>(v);
     if (four && post) return sd <= 32 ? shadow4p_fn<C, 32, B>(v) : shadow4p_fn<C, 64, B>(v);
     if (ext) return sd <= 32 ? ext_fn<C, 32, B>(v) : ext_fn<C, 64, B>(v);
-    if (four) return sd <= 32 ? shadow_fn<C, 32, true, B>(v) : shadow_fn<C, 64, true, B>(v);
+    if constexpr (C) {  // without counters, wide_walk.cu has the four-wide shadow walks
+        if (four) return sd <= 32 ? shadow_fn<C, 32, true, B>(v) : shadow_fn<C, 64, true, B>(v);
+    }
     return sd <= 32 ? shadow_fn<C, 32, false, B>(v) : shadow_fn<C, 64, false, B>(v);
 }
 

@@ -439,12 +439,15 @@ cudaError_t launch_wave_continue(cudaGraphConditionalHandle h, uint32_t* ctr, ui
 }
 
 cudaError_t launch_wave_extend(const WaveArgs& a, bool count, int variant, int stack, int sms, cudaStream_t st) {
+    if (variant >= 3 && !count && a.wide && !a.closest4) return launch_wide_walk(a, true, variant - 3, stack, sms, st);
     if (variant >= 3) return launch_walk(a, count, true, a.closest4 != 0u, variant - 3, stack, sms, st);
     return launch_trav(a, count, true, false, variant, stack, sms, st);
 }
 
 cudaError_t launch_wave_shadow(const WaveArgs& a, bool count, bool four, int variant, int stack, int sms,
                                cudaStream_t st) {
+    if (variant >= 3 && !count && a.wide && four && !a.shadow_post)
+        return launch_wide_walk(a, false, variant - 3, stack, sms, st);
     if (variant >= 3) return launch_walk(a, count, false, four, variant - 3, stack, sms, st);
     return launch_trav(a, count, false, four, variant, stack, sms, st);
 }

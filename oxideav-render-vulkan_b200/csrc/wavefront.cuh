@@ -154,6 +154,9 @@ struct WaveArgs {
     // continuation rays walk the four-wide tree (traversal variants 3-5;
     // the tolerance plan: closest hits equal except near-ties)
     uint32_t closest4 = 0u;
+    // every scene of the launch has its four-wide tree: the walks of
+    // variants 3-5 may use wide_walk.cu
+    uint32_t wide = 0u;
     // four-wide shadow walks of variants 3-5 park leaves until the warp
     // has no node work (same occlusion, fewer mixed node/leaf steps)
     uint32_t shadow_post = 0u;
@@ -190,6 +193,9 @@ cudaError_t launch_wave_shadow(const WaveArgs& a, bool count, bool four, int var
 // (four: the four-wide tree); variant 0..2 targets 6 / 8 / 10 blocks per SM.
 cudaError_t launch_walk(const WaveArgs& a, bool count, bool ext, bool four, int variant, int sd, int sms,
                         cudaStream_t st);
+// wide_walk.cu: closest hits (ext) or shadow rays over the four-wide tree with
+// the reference walk's results; sd: stack entries (32 or 64, the tree's need).
+cudaError_t launch_wide_walk(const WaveArgs& a, bool ext, int variant, int sd, int sms, cudaStream_t st);
 // Graph-resident loop: after an iteration, sets the enclosing while node's
 // condition to "slots still active and fewer than `cap` iterations"; on
 // reaching the bound it sets bit 3 of *err instead. tally[0] += kernels
