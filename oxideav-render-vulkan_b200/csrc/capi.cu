@@ -374,8 +374,9 @@ oxpt_status ensure_wave(oxpt_ctx* c, uint32_t slots, uint32_t jobs, oxd::WaveSta
     size_t sizes[] = {P * 8, P * 16, P * 16, P * 16, P * 16, P * 16, P * 16, P * 16, P * 16, P * 4, P * 4,
                       PJ * 16, P * 4, PJ * 16, PJ * 16, PJ * 16, 64,
                       split ? P * 4 : 0, split ? P * 4 : 0, split ? 13 * P * 16 : 0, P * 4,
-                      (split && jobs <= 32) ? P * 4 : 0, P * 4, PJ * 4, PJ * 4, (size_t)(1u << 17) * 4, PJ * 4};
-    constexpr int NB = 27;
+                      (split && jobs <= 32) ? P * 4 : 0, P * 4, PJ * 4, PJ * 4, (size_t)(1u << 17) * 4, PJ * 4,
+                      split ? P * 4 : 0};
+    constexpr int NB = 28;
     size_t total = 0;
     for (size_t s : sizes) total += align256(s);
     if (slots > c->wave_cap_slots || jobs > c->wave_cap_jobs || total > c->wave_bytes) {
@@ -401,6 +402,7 @@ oxpt_status ensure_wave(oxpt_ctx* c, uint32_t slots, uint32_t jobs, oxd::WaveSta
     q->shade = split ? (uint32_t*)ptr[17] : nullptr;
     q->vslot = split ? (uint32_t*)ptr[18] : nullptr;
     q->vrec = split ? (float4*)ptr[19] : nullptr;
+    q->vlight = split ? (uint32_t*)ptr[27] : nullptr;
     st->item = (unsigned long long*)ptr[0];
     st->seed = (uint4*)ptr[1];
     st->beta = (float4*)ptr[2];

@@ -26,6 +26,7 @@ struct PathCore {
     float prev_pdf;
     uint32_t k;
     bool in_medium;
+    bool sigma_set;  // set by continue_path when it changes sigma
 };
 
 struct Vertex {
@@ -169,116 +170,139 @@ __device__ __forceinline__ int on_path_hit(const Scene& s, const float* sheen, c
     return shade_hit<COUNT>(s, sheen, sobol, smp, pc, hit, hmat, v, shaded);
 }
 
-// NEE job `job` of vertex v (pathtrace.wgsl:1863-1993). True when it arms
-// a shadow ray whose pending contribution is sr->pending.
-__device__ __forceinline__ bool nee_job(const Scene& s, const float* sheen, const PathCore& pc, const Vertex& v,
-                                        uint32_t job, ShadowRay* sr) {
-    const uint32_t strategy = s.P.cfg[1];
-    const bool has_env = s.P.env[2] != 0u;
-    const uint32_t n_elights = s.P.cfg[3], n_punct = s.P.cfg[2];
-    const uint32_t ray_id = pc.k << 16u;
-    bool ok = false;
-    f3 l = sp(0.0f);
-    float tmax = INF;
-    uint32_t rid = ray_id | 0xffffu, skip = NONE;
-    f3 le = sp(0.0f);
-    float pl = -1.0f;
-    const f3 p = v.p;
-    const float4 pl_u = v.pl_u;
-    if (job < n_punct) {
-        LightSample ls = punctual_sample(s, job, p);
-        if (ls.ok) {
-            ok = true;
-            l = ls.l;
-            if (ls.distance >= 0.0f) tmax = ls.distance * (1.0f - 1.0e-4f);
-            rid = ray_id | 0x8000u | (job & 0x7fffu);
-            le = ls.radiance;
-        }
-    } else if (strategy != 2u && (has_env || n_elights > 0u)) {
-        float pe = s.P.fparams[2];
-        if (pl_u.z < pe) {
-            if (has_env) {
-                EnvSample es = env_sample(s, pl_u.x, pl_u.y);
-                if (es.ok && pe * es.pdf > 0.0f) {
-                    ok = true;
-                    l = es.d;
-                    le = es.le;
-                    pl = pe * es.pdf;
-                }
-            }
-        } else if (n_elights > 0u) {
-            float us = pl_u.z;
-            if (pe > 0.0f) us = clampf((pl_u.z - pe) / (1.0f - pe), 0.0f, 0.999999f);
-            uint32_t li = partition_point(s, s.P.offs1[0], n_elights, us, 4u);
-            li = li < n_elights - 1u ? li : n_elights - 1u;
-            uint32_t lslot = tw(s, s.P.offs1[0] + 4u * li + 3u);
-            f3 ta = tri_pos(s, lslot, 0u), tb = tri_pos(s, lslot, 1u), tc = tri_pos(s, lslot, 2u);
-            bool has_target = false;
-            f3 q = sp(0.0f);
-            if (triangle_solid_angle(p, ta, tb, tc) >= MIN_SPHERICAL_SOLID_ANGLE) {
-                f3 sl = sample_spherical_triangle(p, ta, tb, tc, pl_u.x, pl_u.y);
-                if (dot(sl, sl) > 0.0f) {
-                    f3 n = cross(tb - ta, tc - ta);
-                    float dn = dot(sl, n);
-                    if (dn != 0.0f) {
-                        float t = dot(ta - p, n) / dn;
-                        if (t > 0.0f && finite(t)) {
-                            q = p + sl * t;
-                            has_target = true;
-                        }
-                    }
-                }
-            } else {
-                float su = sqrtf(pl_u.x);
-                f3 w3 = mk(1.0f - su, su * (1.0f - pl_u.y), su * pl_u.y);
-                q = ta * w3.x + tb * w3.y + tc * w3.z;
-                has_target = true;
-            }
-            if (has_target) {
-                f3 e1 = tb - ta, e2 = tc - ta, rr = q - ta;
-                float d11 = dot(e1, e1), d12 = dot(e1, e2), d22 = dot(e2, e2);
-                float r1 = dot(rr, e1), r2 = dot(rr, e2);
-                float det = d11 * d22 - d12 * d12;
-                f3 to = q - p;
-                float dist2 = dot(to, to);
-                if (finite(det) && fabsf(det) > 1.17549435e-38f && dist2 > 1.0e-12f) {
-                    float bu = (d22 * r1 - d12 * r2) / det;
-                    float bv = (d11 * r2 - d12 * r1) / det;
-                    f3 lb = vmin(vmax(mk(1.0f - bu - bv, bu, bv), sp(0.0f)), sp(1.0f));
-                    f3 lng = surface(s, lslot, lb).ng;
-                    uint32_t lm = tri_word(s, lslot, 2u);
-                    bool lds = (mat_flags(s, lm) & 4u) != 0u;
-                    float dist = sqrtf(dist2);
-                    f3 ld = to / dist;
-                    float cos_l = -dot(lng, ld);
-                    float tp = tri_pdf(s, li, lslot, p, q);
-                    if ((cos_l > 0.0f || (lds && cos_l < 0.0f)) && tp > 0.0f && finite(tp)) {
-                        ok = true;
-                        l = ld;
-                        le = emission_of(s, lslot, lm, lb);
-                        pl = tp;
-                        tmax = fmaxf(dist * (1.0f - 1.0e-4f), 0.0f);
-                        skip = tri_word(s, lslot, 0u);
-                    }
-                }
-            }
-        }
-    }
-    if (!ok) return false;
-    Eval e = bsdf_eval(sheen, v.bsdf, l);
+// Whether a light in direction `to` (any length) certainly adds nothing at
+// the vertex: below its surface by more than rounding, without transmission.
+// bsdf_eval gives black there; this says so before the light's distance and
+// direction are worked out.
+__device__ __forceinline__ bool surely_dark(const Vertex& v, f3 to) {
+    const Bsdf& b = v.bsdf;
+    return (b.transmission <= 0.0f || b.metallic >= 1.0f) &&
+           dot(b.ng, to) < -1.0e-5f * (fabsf(to.x) + fabsf(to.y) + fabsf(to.z));
+}
+
+// The punctual light `rec`, NEE job `job` of vertex v (pathtrace.wgsl:
+// 1863-1993). True when it arms a shadow ray whose pending contribution is
+// sr->pending.
+__device__ __forceinline__ bool nee_punctual(const Scene& s, const float* sheen, const PathCore& pc, const Vertex& v,
+                                             const ViewTerms& vt, const LightRec& rec, uint32_t job, ShadowRay* sr) {
+    if (surely_dark(v, __float_as_uint(rec.pos.w) == 0u ? -xyz(rec.dir) : xyz(rec.pos) - v.p)) return false;
+    const LightSample ls = punctual_sample(rec, v.p);
+    if (!ls.ok) return false;
+    const Eval e = bsdf_eval_t<false>(sheen, v.bsdf, vt, ls.l);
+    if (is_black(e.f) || is_black(ls.radiance)) return false;
+    sr->pending = clamp_c(s, pc.beta * e.f * ls.radiance);
+    sr->o = spawn(v.p, v.ng, ls.l);
+    sr->d = ls.l;
+    sr->tmax = ls.distance >= 0.0f ? ls.distance * (1.0f - 1.0e-4f) : INF;
+    sr->rid = pc.k << 16u | 0x8000u | (job & 0x7fffu);
+    sr->skip = NONE;
+    return true;
+}
+
+// What the last NEE job of a vertex samples (its direct light by pl_u.z):
+// nothing, the environment or an emissive triangle.
+enum SampledLight : uint32_t { SAMPLED_NONE = 0, SAMPLED_ENV = 1, SAMPLED_AREA = 2 };
+__device__ __forceinline__ uint32_t sampled_light(const Scene& s, float u) {
+    if (s.P.cfg[1] == 2u) return SAMPLED_NONE;
+    if (u < s.P.fparams[2]) return s.P.env[2] != 0u ? SAMPLED_ENV : SAMPLED_NONE;
+    return s.P.cfg[3] > 0u ? SAMPLED_AREA : SAMPLED_NONE;
+}
+
+// The contribution of a light sample with density pl in direction l.
+__device__ __forceinline__ bool nee_weigh(const Scene& s, const float* sheen, const PathCore& pc, const Vertex& v,
+                                          const ViewTerms& vt, f3 l, f3 le, float pl, float tmax, uint32_t skip,
+                                          ShadowRay* sr) {
+    Eval e = bsdf_eval_t<true>(sheen, v.bsdf, vt, l);
     if (is_black(e.f) || is_black(le)) return false;
-    if (pl < 0.0f) {
-        sr->pending = clamp_c(s, pc.beta * e.f * le);
-    } else {
-        float w = strategy == 0u ? power_heuristic(pl, e.pdf) : 1.0f;
-        sr->pending = clamp_c(s, pc.beta * e.f * le * (w / pl));
-    }
-    sr->o = spawn(p, v.ng, l);
+    float w = s.P.cfg[1] == 0u ? power_heuristic(pl, e.pdf) : 1.0f;
+    sr->pending = clamp_c(s, pc.beta * e.f * le * (w / pl));
+    sr->o = spawn(v.p, v.ng, l);
     sr->d = l;
     sr->tmax = tmax;
-    sr->rid = rid;
+    sr->rid = pc.k << 16u | 0xffffu;
     sr->skip = skip;
     return true;
+}
+
+// The last NEE job of vertex v when it samples the environment.
+__device__ __forceinline__ bool nee_env(const Scene& s, const float* sheen, const PathCore& pc, const Vertex& v,
+                                        const ViewTerms& vt, ShadowRay* sr) {
+    const float pe = s.P.fparams[2];
+    const f3 d = env_direction(s, v.pl_u.x, v.pl_u.y);
+    if (surely_dark(v, d)) return false;
+    const EnvSample es = env_sample(s, d);
+    if (!es.ok || !(pe * es.pdf > 0.0f)) return false;
+    return nee_weigh(s, sheen, pc, v, vt, d, es.le, pe * es.pdf, INF, NONE, sr);
+}
+
+// The last NEE job of vertex v when it samples an emissive triangle.
+__device__ __forceinline__ bool nee_area(const Scene& s, const float* sheen, const PathCore& pc, const Vertex& v,
+                                         const ViewTerms& vt, ShadowRay* sr) {
+    const uint32_t n_elights = s.P.cfg[3];
+    const float pe = s.P.fparams[2];
+    const f3 p = v.p;
+    const float4 pl_u = v.pl_u;
+    float us = pl_u.z;
+    if (pe > 0.0f) us = clampf((pl_u.z - pe) / (1.0f - pe), 0.0f, 0.999999f);
+    uint32_t li = partition_point(s, s.P.offs1[0], n_elights, us, 4u);
+    li = li < n_elights - 1u ? li : n_elights - 1u;
+    uint32_t lslot = tw(s, s.P.offs1[0] + 4u * li + 3u);
+    f3 ta = tri_pos(s, lslot, 0u), tb = tri_pos(s, lslot, 1u), tc = tri_pos(s, lslot, 2u);
+    bool has_target = false;
+    f3 q = sp(0.0f);
+    const float omega = triangle_solid_angle(p, ta, tb, tc);
+    if (omega >= MIN_SPHERICAL_SOLID_ANGLE) {
+        f3 sl = sample_spherical_triangle(p, ta, tb, tc, pl_u.x, pl_u.y);
+        if (dot(sl, sl) > 0.0f) {
+            f3 n = cross(tb - ta, tc - ta);
+            float dn = dot(sl, n);
+            if (dn != 0.0f) {
+                float t = dot(ta - p, n) / dn;
+                if (t > 0.0f && finite(t)) {
+                    q = p + sl * t;
+                    has_target = true;
+                }
+            }
+        }
+    } else {
+        float su = sqrtf(pl_u.x);
+        f3 w3 = mk(1.0f - su, su * (1.0f - pl_u.y), su * pl_u.y);
+        q = ta * w3.x + tb * w3.y + tc * w3.z;
+        has_target = true;
+    }
+    if (!has_target) return false;
+    f3 e1 = tb - ta, e2 = tc - ta, rr = q - ta;
+    float d11 = dot(e1, e1), d12 = dot(e1, e2), d22 = dot(e2, e2);
+    float r1 = dot(rr, e1), r2 = dot(rr, e2);
+    float det = d11 * d22 - d12 * d12;
+    f3 to = q - p;
+    float dist2 = dot(to, to);
+    if (!(finite(det) && fabsf(det) > 1.17549435e-38f && dist2 > 1.0e-12f) || surely_dark(v, to)) return false;
+    float bu = (d22 * r1 - d12 * r2) / det;
+    float bv = (d11 * r2 - d12 * r1) / det;
+    f3 lb = vmin(vmax(mk(1.0f - bu - bv, bu, bv), sp(0.0f)), sp(1.0f));
+    f3 lng = surface(s, lslot, lb).ng;
+    uint32_t lm = tri_word(s, lslot, 2u);
+    bool lds = (mat_flags(s, lm) & 4u) != 0u;
+    float dist = sqrtf(dist2);
+    f3 ld = to / dist;
+    float cos_l = -dot(lng, ld);
+    if (!(cos_l > 0.0f || (lds && cos_l < 0.0f))) return false;
+    float tp = tri_pdf(s, li, omega, ta, tb, tc, p, q);
+    if (!(tp > 0.0f && finite(tp))) return false;
+    return nee_weigh(s, sheen, pc, v, vt, ld, emission_of(s, lslot, lm, lb), tp,
+                     fmaxf(dist * (1.0f - 1.0e-4f), 0.0f), tri_word(s, lslot, 0u), sr);
+}
+
+// NEE job `job` of vertex v: punctual light `job`, or the area / environment
+// sample after the last of them.
+__device__ __forceinline__ bool nee_job(const Scene& s, const float* sheen, const PathCore& pc, const Vertex& v,
+                                        uint32_t job, ShadowRay* sr) {
+    const ViewTerms vt = view_terms(sheen, v.bsdf);
+    if (job < s.P.cfg[2]) return nee_punctual(s, sheen, pc, v, vt, light_rec(s, job), job, sr);
+    const uint32_t kind = sampled_light(s, v.pl_u.z);
+    if (kind == SAMPLED_ENV) return nee_env(s, sheen, pc, v, vt, sr);
+    return kind == SAMPLED_AREA && nee_area(s, sheen, pc, v, vt, sr);
 }
 
 // BSDF sampling, medium transition and roulette (pathtrace.wgsl:1999-2039).
@@ -297,6 +321,7 @@ __device__ __forceinline__ bool continue_path(const Scene& s, const float* sheen
         if (v.front && v.atten_dist >= 0.0f) {
             f3 la = vmax(v.atten_color, sp(1.0e-6f));
             pc.sigma = -mk(fm_log(la.x), fm_log(la.y), fm_log(la.z)) / v.atten_dist;
+            pc.sigma_set = true;
             pc.in_medium = true;
         } else {
             pc.in_medium = false;

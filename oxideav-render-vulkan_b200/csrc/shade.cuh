@@ -53,47 +53,68 @@ static __device__ f3 perturb(const Scene& s, uint32_t slot, f3 b, f3 n, float4 t
     return dot(nn, nn) > 0.5f ? nn : n;
 }
 
+// Four words of a material record from word `k` (a multiple of 4): one load
+// where the records are 16-byte aligned (as the host layer lays them out).
+__device__ __forceinline__ float4 mat4(const Scene& s, uint32_t o, uint32_t k) {
+    if ((o & 3u) == 0u) {
+        const uint32_t i = o + k;
+        return (uint64_t)i + 4u <= s.table_words ? __ldg(reinterpret_cast<const float4*>(s.tables + i))
+                                                 : tv4(s, i);
+    }
+    return tv4(s, o + k);
+}
+
 // material() (pathtrace.wgsl:842-902). Slots are sampled in order; an
-// absent slot is white. `m` is the hit's material index.
+// absent slot is white. `m` is the hit's material index. The 13 slots'
+// texture words are loaded together, before any is used: one slot after the
+// other made 13 dependent loads of every hit.
 static __device__ OXD_HEAVY Mat material(const Scene& s, uint32_t slot, uint32_t m, f3 b, f3 sn_in, const Lod& lod, bool flip) {
     f3 sn = flip ? -sn_in : sn_in;
     uint32_t o = mat_off(s, m);
+    uint32_t bound = 0u;
+#pragma unroll
+    for (uint32_t si = 0; si < 13u; si++)
+        if (tw(s, slot_word(s, m, si)) != NONE) bound |= 1u << si;
     float4 tex[13];
-    uint32_t present = 0u;
-    // Fast path: one word per slot tells whether any texture is bound.
 #pragma unroll 1
-    for (uint32_t si = 0; si < 13u; si++) {
-        tex[si] = make_float4(1.f, 1.f, 1.f, 1.f);
-        if (slot_present(s, m, si, slot)) {
-            present |= 1u << si;
-            tex[si] = slot_sample(s, m, si, slot, b, si == S_EMISSIVE ? base_lod() : lod);
-        }
+    for (uint32_t si = 0; si < 13u; si++) tex[si] = make_float4(1.f, 1.f, 1.f, 1.f);
+    uint32_t present = 0u;
+    const uint32_t flags = attr_flags(s, slot);
+    while (bound) {
+        const uint32_t si = (uint32_t)__ffs(bound) - 1u;
+        bound &= bound - 1u;
+        if (!has_uv(s, slot, tw(s, slot_word(s, m, si) + 1u))) continue;
+        present |= 1u << si;
+        tex[si] = slot_sample(s, m, si, slot, b, si == S_EMISSIVE ? base_lod() : lod);
     }
+    float4 w[8];
+#pragma unroll
+    for (uint32_t k = 0; k < 8u; k++) w[k] = mat4(s, o, 4u * k);
     Mat r;
-    float4 col = mul4(tv4(s, o), tex[S_BASE]);
-    if ((attr_flags(s, slot) & F_COLORS) != 0u) col = mul4(col, interp4a(s, slot, 9u, b));
+    float4 col = mul4(w[0], tex[S_BASE]);
+    if ((flags & F_COLORS) != 0u) col = mul4(col, interp4a(s, slot, 9u, b));
     r.base = col;
-    r.metallic = clampf(tf(s, o + 8u) * tex[S_MR].z, 0.0f, 1.0f);
-    r.roughness = clampf(tf(s, o + 9u) * tex[S_MR].y, 0.0f, 1.0f);
+    r.metallic = clampf(w[2].x * tex[S_MR].z, 0.0f, 1.0f);
+    r.roughness = clampf(w[2].y * tex[S_MR].y, 0.0f, 1.0f);
     r.normal = sn;
-    if ((present & (1u << S_NORMAL)) != 0u) r.normal = perturb(s, slot, b, sn, tex[S_NORMAL], tf(s, o + 10u));
-    r.unlit = (tw(s, o + M_FLAGS) & 8u) != 0u;
+    if ((present & (1u << S_NORMAL)) != 0u) r.normal = perturb(s, slot, b, sn, tex[S_NORMAL], w[2].z);
+    r.unlit = (__float_as_uint(w[1].w) & 8u) != 0u;
     r.emission = sp(0.0f);
-    f3 e = tv3(s, o + 4u);
+    f3 e = xyz(w[1]);
     if (!r.unlit && !is_black(e)) r.emission = e * xyz(tex[S_EMISSIVE]);
-    r.ior = tf(s, o + 12u);
-    r.specular = tf(s, o + 13u) * tex[S_SPEC].w;
-    r.specular_color = tv3(s, o + 14u) * xyz(tex[S_SPEC_COLOR]);
-    r.transmission = tf(s, o + 17u) * tex[S_TRANSMISSION].x;
-    r.thickness = tf(s, o + 18u) * tex[S_THICKNESS].y;
-    r.atten_color = tv3(s, o + 19u);
-    r.atten_dist = tf(s, o + 22u);
-    r.clearcoat = tf(s, o + 23u) * tex[S_CC].x;
-    r.cc_rough = tf(s, o + 24u) * tex[S_CC_ROUGH].y;
+    r.ior = w[3].x;
+    r.specular = w[3].y * tex[S_SPEC].w;
+    r.specular_color = mk(w[3].z, w[3].w, w[4].x) * xyz(tex[S_SPEC_COLOR]);
+    r.transmission = w[4].y * tex[S_TRANSMISSION].x;
+    r.thickness = w[4].z * tex[S_THICKNESS].y;
+    r.atten_color = mk(w[4].w, w[5].x, w[5].y);
+    r.atten_dist = w[5].z;
+    r.clearcoat = w[5].w * tex[S_CC].x;
+    r.cc_rough = w[6].x * tex[S_CC_ROUGH].y;
     r.cc_normal = sn;
-    if ((present & (1u << S_CC_NORMAL)) != 0u) r.cc_normal = perturb(s, slot, b, sn, tex[S_CC_NORMAL], tf(s, o + 25u));
-    r.sheen = tv3(s, o + 26u) * xyz(tex[S_SHEEN_COLOR]);
-    r.sheen_rough = tf(s, o + 29u) * tex[S_SHEEN_ROUGH].w;
+    if ((present & (1u << S_CC_NORMAL)) != 0u) r.cc_normal = perturb(s, slot, b, sn, tex[S_CC_NORMAL], w[6].y);
+    r.sheen = mk(w[6].z, w[6].w, w[7].x) * xyz(tex[S_SHEEN_COLOR]);
+    r.sheen_rough = w[7].y * tex[S_SHEEN_ROUGH].w;
     return r;
 }
 
@@ -118,7 +139,6 @@ __device__ __forceinline__ float lambda(float c_in, float a) {
     return (sqrtf(a2 + (1.0f - a2) * c * c) / c - 1.0f) * 0.5f;
 }
 __device__ __forceinline__ float g1(float c, float a) { return 1.0f / (1.0f + lambda(c, a)); }
-__device__ __forceinline__ float g2(float cv, float cl, float a) { return 1.0f / (1.0f + lambda(cv, a) + lambda(cl, a)); }
 __device__ __forceinline__ f3 schlick(f3 f0, float c) {
     float x = 1.0f - clampf(c, 0.0f, 1.0f);
     float k = x * x * x * x * x;
@@ -287,9 +307,33 @@ struct Eval {
     f3 f;
     float pdf;
 };
-static __device__ OXD_HEAVY Eval bsdf_eval(const float* lut, const Bsdf& b, f3 l) {
+// The terms of an evaluation that do not depend on the light's direction,
+// computed once for a vertex that is evaluated against many lights.
+struct ViewTerms {
+    float nv, g_v;    // clamped cosine, 1 + lambda of the specular lobe
+    float cnv, cg_v;  // the clearcoat's
+    float smax, s_v;  // largest sheen weight, 1 - smax x directional albedo
+};
+__device__ __forceinline__ ViewTerms view_terms(const float* lut, const Bsdf& b) {
+    ViewTerms t;
+    t.nv = fmaxf(dot(b.n, b.v), 1.0e-4f);
+    t.g_v = 1.0f + lambda(t.nv, b.alpha);
+    t.cnv = t.cg_v = 0.0f;
+    if (b.clearcoat > 0.0f) {
+        t.cnv = fmaxf(dot(b.ncc, b.v), 1.0e-4f);
+        t.cg_v = 1.0f + lambda(t.cnv, b.cc_alpha);
+    }
+    t.smax = max3(b.sheen);
+    t.s_v = t.smax > 0.0f ? 1.0f - t.smax * sheen_albedo(lut, t.nv, b.sheen_rough) : 1.0f;
+    return t;
+}
+
+// The BSDF's value towards l and, with PDF, the density of sampling it (0
+// without: light samples of punctual lights need no density).
+template <bool PDF>
+static __device__ OXD_HEAVY Eval bsdf_eval_t(const float* lut, const Bsdf& b, const ViewTerms& vt, f3 l) {
     f3 v = b.v, n = b.n;
-    float nv = fmaxf(dot(n, v), 1.0e-4f);
+    const float nv = vt.nv;
     if (dot(b.ng, l) > 0.0f) {
         float nl = dot(n, l);
         f3 h = nrm(v + l);
@@ -300,29 +344,29 @@ static __device__ OXD_HEAVY Eval bsdf_eval(const float* lut, const Bsdf& b, f3 l
         if (nl > 0.0f) {
             f3 fd = fresnel_d(b, vh);
             f3 fm = schlick(b.base, vh);
-            float spec_c = d_ggx(nh, b.alpha) * g2(nv, nl, b.alpha) / (4.0f * nv * nl);
+            float spec_c = d_ggx(nh, b.alpha) * (1.0f / (vt.g_v + lambda(nl, b.alpha))) / (4.0f * nv * nl);
             float m = b.metallic;
             float diff_k = (1.0f - m) * (1.0f - b.transmission) * (1.0f - b.specular * max3(fd)) / PI;
             f3 layer = spec_c * ((1.0f - m) * b.specular * fd + m * fm) + diff_k * b.base;
-            float smax = max3(b.sheen);
-            if (smax > 0.0f) {
-                float scale = fminf(1.0f - smax * sheen_albedo(lut, nv, b.sheen_rough),
-                                    1.0f - smax * sheen_albedo(lut, nl, b.sheen_rough));
+            if (vt.smax > 0.0f) {
+                float scale = fminf(vt.s_v, 1.0f - vt.smax * sheen_albedo(lut, nl, b.sheen_rough));
                 float sh = d_charlie(nh, b.sheen_alpha) * v_neubelt(nl, nv);
                 layer = layer * scale + b.sheen * sh;
             }
             f = layer * (1.0f - b.w_cc);
-            pdf += (b.p0 + b.p4) * nl / PI;
-            pdf += b.p1 * vndf_reflect_pdf(n, v, h, b.alpha);
+            if (PDF) {
+                pdf += (b.p0 + b.p4) * nl / PI;
+                pdf += b.p1 * vndf_reflect_pdf(n, v, h, b.alpha);
+            }
         }
         if (b.clearcoat > 0.0f) {
-            float cnv = fmaxf(dot(b.ncc, v), 1.0e-4f);
             float cnl = dot(b.ncc, l);
             if (cnl > 0.0f) {
                 float cnh = dot(b.ncc, h);
-                float c = b.w_cc * d_ggx(cnh, b.cc_alpha) * g2(cnv, cnl, b.cc_alpha) / (4.0f * cnv * cnl);
+                float c = b.w_cc * d_ggx(cnh, b.cc_alpha) * (1.0f / (vt.cg_v + lambda(cnl, b.cc_alpha))) /
+                          (4.0f * vt.cnv * cnl);
                 f = f + sp(c);
-                pdf += b.p3 * vndf_reflect_pdf(b.ncc, v, h, b.cc_alpha);
+                if (PDF) pdf += b.p3 * vndf_reflect_pdf(b.ncc, v, h, b.cc_alpha);
             }
         }
         return {f * fmaxf(nl, 0.0f), pdf};
@@ -330,18 +374,16 @@ static __device__ OXD_HEAVY Eval bsdf_eval(const float* lut, const Bsdf& b, f3 l
     if (b.transmission <= 0.0f || b.metallic >= 1.0f) return {sp(0.0f), 0.0f};
     float nl = -dot(n, l);
     if (nl <= 0.0f) return {sp(0.0f), 0.0f};
-    float smax = max3(b.sheen);
-    float sheen_scale = smax > 0.0f ? 1.0f - smax * sheen_albedo(lut, nv, b.sheen_rough) : 1.0f;
-    float w = (1.0f - b.metallic) * b.transmission * (1.0f - b.w_cc) * sheen_scale;
-    float val, pdf_t;
+    float w = (1.0f - b.metallic) * b.transmission * (1.0f - b.w_cc) * vt.s_v;
+    float val, pdf_t = 0.0f;
     if (b.thin) {
         f3 lm = l + n * (2.0f * nl);
         f3 h = nrm(v + lm);
         float vh = dot(v, h), nh = dot(n, h);
         if (vh <= 0.0f || nh <= 0.0f) return {sp(0.0f), 0.0f};
         float fd = b.specular * max3(fresnel_d(b, vh));
-        val = d_ggx(nh, b.alpha) * g2(nv, nl, b.alpha) / (4.0f * nv * nl) * (1.0f - fd);
-        pdf_t = vndf_reflect_pdf(n, v, h, b.alpha);
+        val = d_ggx(nh, b.alpha) * (1.0f / (vt.g_v + lambda(nl, b.alpha))) / (4.0f * nv * nl) * (1.0f - fd);
+        if (PDF) pdf_t = vndf_reflect_pdf(n, v, h, b.alpha);
     } else {
         float ei = b.eta_i, et = b.eta_t;
         f3 h = nrm(-(ei * v + et * l));
@@ -352,11 +394,17 @@ static __device__ OXD_HEAVY Eval bsdf_eval(const float* lut, const Bsdf& b, f3 l
         if (fabsf(denom) < 1.0e-6f) return {sp(0.0f), 0.0f};
         float d = d_ggx(nh, b.alpha);
         float fd = b.specular * max3(fresnel_d(b, vh));
-        float jac = et * et * fabsf(lh) / (denom * denom);
-        val = vh * fabsf(lh) * d * g2(nv, nl, b.alpha) * et * et * (1.0f - fd) / (nv * nl * denom * denom);
-        pdf_t = g1(nv, b.alpha) * vh * d / nv * jac;
+        val = vh * fabsf(lh) * d * (1.0f / (vt.g_v + lambda(nl, b.alpha))) * et * et * (1.0f - fd) /
+              (nv * nl * denom * denom);
+        if (PDF) {
+            float jac = et * et * fabsf(lh) / (denom * denom);
+            pdf_t = g1(nv, b.alpha) * vh * d / nv * jac;
+        }
     }
     return {b.base * (w * val * nl), b.p2 * pdf_t};
+}
+static __device__ OXD_HEAVY Eval bsdf_eval(const float* lut, const Bsdf& b, f3 l) {
+    return bsdf_eval_t<true>(lut, b, view_terms(lut, b), l);
 }
 
 struct BSample {
@@ -432,12 +480,20 @@ struct LightSample {
     float distance;
     f3 radiance;
 };
-static __device__ LightSample punctual_sample(const Scene& s, uint32_t j, f3 p) {
-    uint32_t o = s.P.offs0[3] + 16u * j;
+// A punctual light's record: position and kind, direction and range, colour
+// x intensity, cone scale and offset.
+struct LightRec {
+    float4 pos, dir, base, cone;
+};
+__device__ __forceinline__ LightRec light_rec(const Scene& s, uint32_t j) {
+    const uint32_t o = s.P.offs0[3] + 16u * j;
+    return {tv4(s, o), tv4(s, o + 4u), tv4(s, o + 8u), tv4(s, o + 12u)};
+}
+static __device__ LightSample punctual_sample(const LightRec& rec, f3 p) {
     LightSample r;
     r.ok = false;
-    uint32_t kind = tw(s, o + 3u);
-    f3 base = tv3(s, o + 8u), dir = tv3(s, o + 4u);
+    uint32_t kind = __float_as_uint(rec.pos.w);
+    f3 base = xyz(rec.base), dir = xyz(rec.dir);
     if (kind == 0u) {
         r.ok = true;
         r.l = -dir;
@@ -445,20 +501,20 @@ static __device__ LightSample punctual_sample(const Scene& s, uint32_t j, f3 p) 
         r.radiance = base;
         return r;
     }
-    f3 to = tv3(s, o) - p;
+    f3 to = xyz(rec.pos) - p;
     float d2 = dot(to, to);
     if (!(d2 > 1.0e-12f)) return r;
     float d = sqrtf(d2);
     f3 l = to / d;
     float att = 1.0f / d2;
-    float range = tf(s, o + 7u);
+    float range = rec.dir.w;
     if (range > 0.0f) {
         float x = d / range;
         att *= clampf(1.0f - x * x * x * x, 0.0f, 1.0f);
     }
     if (kind == 2u) {
         float cd = dot(dir, -l);
-        float a = clampf(cd * tf(s, o + 12u) + tf(s, o + 13u), 0.0f, 1.0f);
+        float a = clampf(cd * rec.cone.x + rec.cone.y, 0.0f, 1.0f);
         att *= a * a;
     }
     if (att <= 0.0f) return r;
@@ -516,10 +572,10 @@ static __device__ OXD_HEAVY f3 sample_spherical_triangle(f3 p, f3 a0, f3 b0, f3 
     if (dot(cb_perp, cb_perp) > 0.0f) d = z * b + w * cb_perp;
     return nrm_any(d);
 }
-static __device__ float tri_pdf(const Scene& s, uint32_t li, uint32_t slot, f3 p, f3 q) {
-    f3 a = tri_pos(s, slot, 0u), b = tri_pos(s, slot, 1u), c = tri_pos(s, slot, 2u);
+// Density of sampling point q of the emissive triangle a, b, c (light li)
+// from p, where it subtends the solid angle omega.
+static __device__ float tri_pdf(const Scene& s, uint32_t li, float omega, f3 a, f3 b, f3 c, f3 p, f3 q) {
     float sel = (1.0f - s.P.fparams[2]) * tf(s, s.P.offs1[0] + 4u * li + 1u);
-    float omega = triangle_solid_angle(p, a, b, c);
     if (omega >= MIN_SPHERICAL_SOLID_ANGLE) return sel / omega;
     f3 cr = cross(b - a, c - a);
     float len = sqrtf(dot(cr, cr));
@@ -529,6 +585,10 @@ static __device__ float tri_pdf(const Scene& s, uint32_t li, uint32_t slot, f3 p
     float cs = fabsf(dot(cr, to) / (len * sqrtf(d2)));
     if (cs <= 0.0f) return 0.0f;
     return sel * d2 / (0.5f * len * cs);
+}
+static __device__ float tri_pdf(const Scene& s, uint32_t li, uint32_t slot, f3 p, f3 q) {
+    f3 a = tri_pos(s, slot, 0u), b = tri_pos(s, slot, 1u), c = tri_pos(s, slot, 2u);
+    return tri_pdf(s, li, triangle_solid_angle(p, a, b, c), a, b, c, p, q);
 }
 struct Texel {
     uint32_t x, y;
@@ -553,14 +613,8 @@ __device__ __forceinline__ float env_pdf_at(const Scene& s, const Texel& t) {
     uint32_t w = s.P.env[0], h = s.P.env[1];
     return tf(s, s.P.offs2[0] + t.y * w + t.x) * (float)(w * h) / (2.0f * PI * PI * t.st);
 }
-struct EnvSample {
-    bool ok;
-    f3 d, le;
-    float pdf;
-};
-static __device__ OXD_HEAVY EnvSample env_sample(const Scene& s, float u0, float u1) {
-    EnvSample r;
-    r.ok = false;
+// The environment direction at (u0, u1) of its distribution, and its sample.
+static __device__ OXD_HEAVY f3 env_direction(const Scene& s, float u0, float u1) {
     uint32_t w = s.P.env[0], h = s.P.env[1];
     uint32_t marg = s.P.offs1[2];
     uint32_t pp = partition_point(s, marg, h + 1u, u0, 1u);
@@ -575,12 +629,20 @@ static __device__ OXD_HEAVY EnvSample env_sample(const Scene& s, float u0, float
     float phi = 2.0f * PI * (u - 0.5f);
     float th = PI * v;
     float st = fm_sin(th), ct = fm_cos(th);
-    f3 d = mk(st * fm_sin(phi), ct, -st * fm_cos(phi));
+    return mk(st * fm_sin(phi), ct, -st * fm_cos(phi));
+}
+struct EnvSample {
+    bool ok;
+    f3 le;
+    float pdf;
+};
+static __device__ EnvSample env_sample(const Scene& s, f3 d) {
+    EnvSample r;
+    r.ok = false;
     Texel t = env_texel(s, d);
     float pdf = env_pdf_at(s, t);
     if (pdf <= 0.0f || !finite(pdf)) return r;
     r.ok = true;
-    r.d = d;
     r.le = env_radiance_at(s, t);
     r.pdf = pdf;
     return r;

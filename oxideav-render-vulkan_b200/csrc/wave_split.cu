@@ -18,6 +18,8 @@
 // continuation ray finds.
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "path.cuh"
 #include "shade.cuh"
@@ -43,16 +45,10 @@ __device__ __forceinline__ uint32_t append1(uint32_t* ctr) {
     if (g.thread_rank() == 0) base = atomicAdd(ctr, g.size());
     return g.shfl(base, 0) + g.thread_rank();
 }
-__device__ __forceinline__ unsigned long long fetch1(unsigned long long* ctr) {
-    cg::coalesced_group g = cg::coalesced_threads();
-    unsigned long long base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(ctr, (unsigned long long)g.size());
-    return g.shfl(base, 0) + g.thread_rank();
-}
-
+// What split_shade needs of a path (its medium's extinction stays in memory).
 __device__ __forceinline__ void load_state(const WaveArgs& a, uint32_t i, PathCore* pc, Sampler* smp) {
     uint4 sd = a.st.seed[i];
-    float4 b = a.st.beta[i], r = a.st.rad[i], d = a.st.dir[i], pp = a.st.prev[i], sg = a.st.sigma[i];
+    float4 b = a.st.beta[i], r = a.st.rad[i], d = a.st.dir[i], pp = a.st.prev[i];
     smp->pixel_seed = sd.x;
     smp->index = sd.y;
     smp->path_seed = sd.z;
@@ -63,18 +59,22 @@ __device__ __forceinline__ void load_state(const WaveArgs& a, uint32_t i, PathCo
     pc->in_medium = (__float_as_uint(r.w) & 4u) != 0u;
     pc->d = xyz(d);
     pc->prev_pos = xyz(pp);
-    pc->sigma = xyz(sg);
+    pc->sigma = sp(0.0f);
+    pc->sigma_set = false;
 }
 
-__device__ __forceinline__ void save_state(const WaveArgs& a, uint32_t i, const PathCore& pc, const Sampler& smp,
-                                           uint32_t stage) {
-    a.st.seed[i] = make_uint4(smp.pixel_seed, smp.index, smp.path_seed, pc.k);
-    a.st.beta[i] = make_float4(pc.beta.x, pc.beta.y, pc.beta.z, pc.prev_pdf);
+__device__ __forceinline__ void save_rad(const WaveArgs& a, uint32_t i, const PathCore& pc, uint32_t stage) {
     a.st.rad[i] = make_float4(pc.radiance.x, pc.radiance.y, pc.radiance.z,
                               __uint_as_float(stage | (pc.in_medium ? 4u : 0u)));
+}
+
+// A path that goes on: only what a bounce changes is written. A path that
+// ends needs no more than save_rad.
+__device__ __forceinline__ void save_ray(const WaveArgs& a, uint32_t i, const PathCore& pc, f3 o) {
+    save_rad(a, i, pc, ST_TRACING);
+    a.st.beta[i] = make_float4(pc.beta.x, pc.beta.y, pc.beta.z, pc.prev_pdf);
     a.st.dir[i] = make_float4(pc.d.x, pc.d.y, pc.d.z, 0.0f);
-    a.st.prev[i] = make_float4(pc.prev_pos.x, pc.prev_pos.y, pc.prev_pos.z, 0.0f);
-    a.st.sigma[i] = make_float4(pc.sigma.x, pc.sigma.y, pc.sigma.z, 0.0f);
+    a.st.org[i] = make_float4(o.x, o.y, o.z, 0.0f);
 }
 
 __device__ __forceinline__ Hit load_hit(const WaveArgs& a, uint32_t i, uint32_t* hmat) {
@@ -196,82 +196,148 @@ __device__ __forceinline__ void nrc_finish(const WaveArgs& a, uint32_t i, const 
 
 }  // namespace
 
-template <bool COUNT, bool BATCH>
-__global__ void __launch_bounds__(128, 4) split_logic(const __grid_constant__ WaveArgs a) {
-    __shared__ uint32_t s_sobol[128];
-    {
-        const Scene& s0 = tables_of<BATCH>(a);
-        for (uint32_t i = threadIdx.x; i < 128u; i += blockDim.x) s_sobol[i] = tw(s0, s0.P.offs0[0] + i);
-    }
-    __syncthreads();
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.slots) return;
+// What split_logic found at a slot.
+enum LogicOutcome : uint32_t { SLOT_SURFACE, SLOT_FREED, SLOT_EMPTY };
+
+// Adds the slot's NEE terms and takes its path past its ray: a surface hit to
+// shade, or a finished path, whose result is stored. What every slot reads is
+// loaded first, together.
+template <bool BATCH>
+__device__ __forceinline__ uint32_t logic_slot(const WaveArgs& a, uint32_t i) {
     const uint32_t J = a.jobs;
     PathCore pc;
-    Sampler smp;
-    uint32_t stage = __float_as_uint(a.st.rad[i].w) & 3u;
-    bool need_new = stage == ST_EMPTY;
-    if (!need_new) {
-        const Scene& s = slot_scene<BATCH>(a, i);
-        load_state(a, i, &pc, &smp);
-        uint32_t n = a.st.nee_n[i];
-        if (a.st.vis) {
-            // The unoccluded jobs' contributions, in job order.
-            uint32_t m = n ? a.st.vis[i] : 0u;
-            while (m) {
-                uint32_t j = __ffs(m) - 1u;
-                m &= m - 1u;
-                if (j < n) pc.radiance = pc.radiance + xyz(a.st.pend[(uint64_t)i * J + j]);
-            }
-        } else {
-            for (uint32_t j = 0; j < n; j++) {
-                float4 pe = a.st.pend[(uint64_t)i * J + j];
-                if (pe.w == 2.0f) pc.radiance = pc.radiance + xyz(pe);
-            }
+    const float4 rad = a.st.rad[i];
+    const uint32_t n = a.st.nee_n[i], vis = a.st.vis ? a.st.vis[i] : 0u;
+    const uint4 h = a.st.hit[i];
+    const unsigned long long item = a.st.item[i];
+    const uint32_t stage = __float_as_uint(rad.w) & 3u;
+    if (stage == ST_EMPTY) return SLOT_EMPTY;
+    pc.radiance = xyz(rad);
+    pc.in_medium = (__float_as_uint(rad.w) & 4u) != 0u;
+    if (a.st.vis) {
+        // The unoccluded jobs' contributions, in job order.
+        uint32_t m = n ? vis : 0u;
+        while (m) {
+            uint32_t j = __ffs(m) - 1u;
+            m &= m - 1u;
+            if (j < n) pc.radiance = pc.radiance + xyz(a.st.pend[(uint64_t)i * J + j]);
         }
-        if (n) a.st.nee_n[i] = 0u;
-        int r = PATH_DONE;
-        if (stage == ST_TRACING) {
-            uint32_t hmat;
-            Hit hit = load_hit(a, i, &hmat);
-            r = after_ray(s, pc, hit.slot != NONE, hit);
+    } else {
+        for (uint32_t j = 0; j < n; j++) {
+            float4 pe = a.st.pend[(uint64_t)i * J + j];
+            if (pe.w == 2.0f) pc.radiance = pc.radiance + xyz(pe);
         }
-        if (r == PATH_SURFACE) {
-            save_state(a, i, pc, smp, ST_TRACING);
-            a.q.shade[append1(&a.ctr[3])] = i;
-            append1(&a.ctr[2]);
-            return;
-        }
-        a.out[a.st.item[i]] = path_result(pc, r != PATH_UNCOVERED);
-        if (a.nrc.on) nrc_finish(a, i, pc);
-        need_new = true;
     }
-    unsigned long long item = fetch1(a.work);
-    if (item < a.total) {
-        uint32_t f = BATCH ? frame_of1(a, item) : 0u;
-        const Scene& s = BATCH ? a.frames[f].s : a.s;
-        unsigned long long local = BATCH ? item - a.frames[f].base : item;
-        uint32_t npix = BATCH ? a.frames[f].npix : a.npix;
-        uint32_t y0 = BATCH ? a.frames[f].y0 : a.y0, first = BATCH ? a.frames[f].first : a.first;
-        uint32_t it = (uint32_t)(local / npix);
-        uint32_t q = (uint32_t)(local - (unsigned long long)it * npix);
-        uint32_t yy = q / s.P.dims[0];
-        f3 o = start_path(s, s_sobol, q - yy * s.P.dims[0], y0 + yy, first + it, &smp, &pc);
-        a.st.item[i] = item;
-        if (BATCH) a.st.frame[i] = f;
-        if (a.nrc.on) {
-            a.nrc.s_tidx[i] = NONE;
-            a.nrc.s_tail[i] = NONE;
+    if (n) a.st.nee_n[i] = 0u;
+    int r = PATH_DONE;
+    if (stage == ST_TRACING) {
+        r = PATH_SURFACE;
+        if (h.x == NONE || pc.in_medium) {
+            const float4 b = a.st.beta[i], d = a.st.dir[i];
+            pc.beta = xyz(b);
+            pc.prev_pdf = b.w;
+            pc.d = xyz(d);
+            pc.k = a.st.seed[i].w;
+            if (pc.in_medium) pc.sigma = xyz(a.st.sigma[i]);
+            Hit hit;
+            hit.t = __uint_as_float(h.y);
+            r = after_ray(slot_scene<BATCH>(a, i), pc, h.x != NONE, hit);
+            if (r == PATH_SURFACE) a.st.beta[i] = make_float4(pc.beta.x, pc.beta.y, pc.beta.z, pc.prev_pdf);
         }
-        save_state(a, i, pc, smp, ST_TRACING);
-        a.st.org[i] = make_float4(o.x, o.y, o.z, 0.0f);
-        a.q.ext[append1(&a.ctr[0])] = i;
-        append1(&a.ctr[2]);
-        if (COUNT) atomicAdd(a.counters + C_PATHS, 1ull);
-    } else if (stage != ST_EMPTY) {
-        float4 r = a.st.rad[i];
-        r.w = __uint_as_float(ST_EMPTY);
-        a.st.rad[i] = r;
+    }
+    if (r == PATH_SURFACE) {
+        save_rad(a, i, pc, ST_TRACING);
+        return SLOT_SURFACE;
+    }
+    a.out[item] = path_result(pc, r != PATH_UNCOVERED);
+    if (a.nrc.on) nrc_finish(a, i, pc);
+    return SLOT_FREED;
+}
+
+// Starts the path of launch item `item` in slot i.
+template <bool BATCH>
+__device__ __forceinline__ void start_slot(const WaveArgs& a, uint32_t i, unsigned long long item,
+                                           const uint32_t* s_sobol) {
+    PathCore pc;
+    Sampler smp;
+    uint32_t f = BATCH ? frame_of1(a, item) : 0u;
+    const Scene& s = BATCH ? a.frames[f].s : a.s;
+    unsigned long long local = BATCH ? item - a.frames[f].base : item;
+    uint32_t npix = BATCH ? a.frames[f].npix : a.npix;
+    uint32_t y0 = BATCH ? a.frames[f].y0 : a.y0, first = BATCH ? a.frames[f].first : a.first;
+    uint32_t it = (uint32_t)(local / npix);
+    uint32_t q = (uint32_t)(local - (unsigned long long)it * npix);
+    uint32_t yy = q / s.P.dims[0];
+    f3 o = start_path(s, s_sobol, q - yy * s.P.dims[0], y0 + yy, first + it, &smp, &pc);
+    a.st.item[i] = item;
+    if (BATCH) a.st.frame[i] = f;
+    if (a.nrc.on) {
+        a.nrc.s_tidx[i] = NONE;
+        a.nrc.s_tail[i] = NONE;
+    }
+    a.st.seed[i] = make_uint4(smp.pixel_seed, smp.index, smp.path_seed, pc.k);
+    save_ray(a, i, pc, o);
+}
+
+constexpr uint32_t LOGIC_THREADS = 256u;
+
+// One thread per slot; a block asks for its places in the queues and its new
+// items once. Each warp asking for itself made five atomics a warp on one
+// 64-byte line the kernel's bound (4.2 M slots: 365 us whether it moved 1.3
+// or 0.6 GB).
+template <bool COUNT, bool BATCH>
+__global__ void __launch_bounds__(LOGIC_THREADS, 4) split_logic(const __grid_constant__ WaveArgs a) {
+    constexpr uint32_t WARPS = LOGIC_THREADS / 32u;
+    __shared__ uint32_t s_sobol[128];
+    __shared__ uint32_t s_surface[WARPS], s_free[WARPS];
+    __shared__ uint32_t s_shade_at, s_ext_at;
+    __shared__ unsigned long long s_item_at;
+    const uint32_t i = blockIdx.x * LOGIC_THREADS + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (i == 0u) a.ctr[11] = a.ctr[12] = 0u;  // counted by split_shade
+    const uint32_t out = i < a.slots ? logic_slot<BATCH>(a, i) : (uint32_t)SLOT_EMPTY;
+    const bool surface = out == SLOT_SURFACE, free_slot = !surface && i < a.slots;
+    const unsigned below = (1u << lane) - 1u;
+    const unsigned ms = __ballot_sync(0xffffffffu, surface), mf = __ballot_sync(0xffffffffu, free_slot);
+    if (lane == 0u) {
+        s_surface[warp] = __popc(ms);
+        s_free[warp] = __popc(mf);
+    }
+    __syncthreads();
+    uint32_t surfaces = 0u, frees = 0u, my_surface = __popc(ms & below), my_free = __popc(mf & below);
+#pragma unroll
+    for (uint32_t w = 0; w < WARPS; w++) {
+        if (w == warp) {
+            my_surface += surfaces;
+            my_free += frees;
+        }
+        surfaces += s_surface[w];
+        frees += s_free[w];
+    }
+    if (threadIdx.x == 0u) {
+        uint32_t starts = 0u;
+        if (frees) {
+            s_item_at = atomicAdd(a.work, (unsigned long long)frees);
+            const unsigned long long left = s_item_at < a.total ? a.total - s_item_at : 0ull;
+            starts = left < frees ? (uint32_t)left : frees;
+            if (starts) s_ext_at = atomicAdd(&a.ctr[0], starts);
+        }
+        if (surfaces) s_shade_at = atomicAdd(&a.ctr[3], surfaces);
+        if (surfaces + starts) atomicAdd(&a.ctr[2], surfaces + starts);
+        if (COUNT && starts) atomicAdd(a.counters + C_PATHS, (unsigned long long)starts);
+    }
+    if (frees) {
+        const Scene& s0 = tables_of<BATCH>(a);
+        for (uint32_t k = threadIdx.x; k < 128u; k += LOGIC_THREADS) s_sobol[k] = tw(s0, s0.P.offs0[0] + k);
+    }
+    __syncthreads();
+    if (surface) a.q.shade[s_shade_at + my_surface] = i;
+    if (!free_slot) return;
+    const unsigned long long item = s_item_at + my_free;
+    if (item < a.total) {
+        start_slot<BATCH>(a, i, item, s_sobol);
+        a.q.ext[s_ext_at + my_free] = i;
+    } else if (out != SLOT_EMPTY) {
+        a.st.rad[i].w = __uint_as_float(ST_EMPTY);
     }
 }
 
@@ -287,7 +353,10 @@ __global__ void __launch_bounds__(128, MINB) split_shade(const __grid_constant__
     __syncthreads();
     const uint32_t n = *((volatile uint32_t*)&a.ctr[3]);
     unsigned long long shaded = 0;
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+    for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < n; q0 += gridDim.x * blockDim.x) {
+        __syncthreads();  // the block's warps fetch the same code together
+        uint32_t q = q0 + threadIdx.x;
+        if (q >= n) continue;
         uint32_t i = a.q.shade[q];
         const Scene& s = slot_scene<BATCH>(a, i);
         PathCore pc;
@@ -298,7 +367,7 @@ __global__ void __launch_bounds__(128, MINB) split_shade(const __grid_constant__
         Vertex vx;
         int r = shade_hit<COUNT>(s, s_sheen, s_sobol, smp, pc, hit, hmat, &vx, &shaded);
         if (r != PATH_VERTEX) {
-            save_state(a, i, pc, smp, ST_ENDING);
+            save_rad(a, i, pc, ST_ENDING);
             continue;
         }
         bool spread_ok = true;
@@ -334,7 +403,7 @@ __global__ void __launch_bounds__(128, MINB) split_shade(const __grid_constant__
                 }
             }
             a.st.nee_n[i] = 0u;
-            save_state(a, i, pc, smp, ST_ENDING);
+            save_rad(a, i, pc, ST_ENDING);
             continue;
         }
         if (a.nrc.on && pc.k >= a.nrc.query_k && tail == NONE && spread_ok) {
@@ -351,7 +420,7 @@ __global__ void __launch_bounds__(128, MINB) split_shade(const __grid_constant__
                     a.nrc.q_item[q] = a.st.item[i];
                 }
                 a.st.nee_n[i] = 0u;
-                save_state(a, i, pc, smp, ST_ENDING);
+                save_rad(a, i, pc, ST_ENDING);
                 continue;
             }
             a.nrc.s_tail[i] = a.nrc.suffix ? pc.k + a.nrc.suffix : 0xfffffffeu;
@@ -370,144 +439,181 @@ __global__ void __launch_bounds__(128, MINB) split_shade(const __grid_constant__
         uint32_t v = append1(&a.ctr[4]);
         put_vertex(a, v, vx, pc, smp.path_seed);
         a.q.vslot[v] = i;
-        a.st.nee_n[i] = BATCH ? s.P.cfg[2] + 1u : a.jobs;
+        const uint32_t jobs = BATCH ? s.P.cfg[2] + 1u : a.jobs;
+        a.st.nee_n[i] = jobs;
+        if (a.st.vis) a.st.vis[i] = 0u;
+        const uint32_t kind = sampled_light(s, vx.pl_u.z);
+        if (kind == SAMPLED_ENV) a.q.vlight[append1(&a.ctr[11])] = v;
+        else if (kind == SAMPLED_AREA) a.q.vlight[a.vcap - 1u - append1(&a.ctr[12])] = v;
+        else if (!a.st.vis) a.st.pend[(uint64_t)i * a.jobs + jobs - 1u] = make_float4(0.f, 0.f, 0.f, 0.f);
         f3 o;
         if (continue_path(s, s_sheen, s_sobol, smp, pc, vx, &o)) {
-            save_state(a, i, pc, smp, ST_TRACING);
-            a.st.org[i] = make_float4(o.x, o.y, o.z, 0.0f);
+            a.st.seed[i].w = pc.k;
+            a.st.prev[i] = make_float4(pc.prev_pos.x, pc.prev_pos.y, pc.prev_pos.z, 0.0f);
+            if (pc.sigma_set) a.st.sigma[i] = make_float4(pc.sigma.x, pc.sigma.y, pc.sigma.z, 0.0f);
+            save_ray(a, i, pc, o);
             a.q.ext[append1(&a.ctr[0])] = i;
         } else {
-            save_state(a, i, pc, smp, ST_ENDING);
+            save_rad(a, i, pc, ST_ENDING);
         }
     }
     if (COUNT && shaded) atomicAdd(a.counters + C_SHADED, shaded);
 }
 
-template <bool COUNT, int MINB, bool BATCH>
-__global__ void __launch_bounds__(128, MINB) split_nee(const __grid_constant__ WaveArgs a) {
-    __shared__ float s_sheen[512];
-    {
-        const Scene& s0 = tables_of<BATCH>(a);
-        for (uint32_t i = threadIdx.x; i < 512u; i += blockDim.x) s_sheen[i] = tf(s0, s0.P.offs0[1] + i);
+constexpr uint32_t NEE_THREADS = 256u;
+constexpr uint32_t NEE_LIGHTS = 64u;  // punctual lights the vertex-major kernel keeps in shared memory
+
+// Stores NEE job j of `slot`: queues its shadow ray, and its contribution
+// (without visibility masks, also that there is none).
+__device__ __forceinline__ void put_job(const WaveArgs& a, uint32_t slot, uint32_t j, uint32_t path_seed, bool queued,
+                                        const ShadowRay& sr) {
+    float4 pe = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (queued) {
+        pe = make_float4(sr.pending.x, sr.pending.y, sr.pending.z, 1.0f);
+        uint32_t q = append1(&a.ctr[1]);
+        a.q.sh_o[q] = make_float4(sr.o.x, sr.o.y, sr.o.z, sr.tmax);
+        a.q.sh_d[q] = make_float4(sr.d.x, sr.d.y, sr.d.z, __uint_as_float(sr.skip));
+        a.q.sh_m[q] = make_uint4(slot, j, sr.rid, path_seed);
     }
-    __syncthreads();
-    const uint32_t nv = *((volatile uint32_t*)&a.ctr[4]);
-    const uint64_t total = (uint64_t)nv * a.jobs;
-    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-         t += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t j = (uint32_t)(t / nv);
-        uint32_t v = (uint32_t)(t - (uint64_t)j * nv);
-        uint32_t slot = a.q.vslot[v];
-        const Scene& s = slot_scene<BATCH>(a, slot);
-        if (BATCH && j > s.P.cfg[2]) continue;  // beyond this scene's NEE jobs (its nee_n stops short)
-        Vertex vx;
-        PathCore pc;
-        uint32_t path_seed;
-        get_vertex(a, v, &vx, &pc, &path_seed);
-        ShadowRay sr;
-        float4 pe = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (a.st.vis && j == 0u) a.st.vis[slot] = 0u;
-        bool queued = nee_job(s, s_sheen, pc, vx, j, &sr);
-        if (queued) {
-            pe = make_float4(sr.pending.x, sr.pending.y, sr.pending.z, 1.0f);
-            uint32_t q = append1(&a.ctr[1]);
-            a.q.sh_o[q] = make_float4(sr.o.x, sr.o.y, sr.o.z, sr.tmax);
-            a.q.sh_d[q] = make_float4(sr.d.x, sr.d.y, sr.d.z, __uint_as_float(sr.skip));
-            a.q.sh_m[q] = make_uint4(slot, j, sr.rid, path_seed);
-        }
-        if (queued || !a.st.vis) a.st.pend[(uint64_t)slot * a.jobs + j] = pe;
-    }
+    if (queued || !a.st.vis) a.st.pend[(uint64_t)slot * a.jobs + j] = pe;
 }
 
-// The same NEE jobs vertex-major: one thread per vertex loads its record
-// once and runs every job in order, so the lanes of a warp still evaluate
-// the same light together while the vertex array is read once instead of
-// once per job. Each (vertex, job) computes what split_nee computes; only
-// the order of the shadow queue changes (warp-sized runs per light).
-template <bool COUNT, int MINB, bool BATCH>
-__global__ void __launch_bounds__(128, MINB) split_nee_v(const __grid_constant__ WaveArgs a) {
+// The vertices' NEE jobs, one kind of light after the other: environment
+// samples, emissive-triangle samples (lists made by split_shade, so their
+// warps are full), then punctual lights. All warps of the grid then run the
+// same few kilobytes of code at a time; with one thread doing every job of a
+// vertex in order, 75% of the warps' time went to fetching instructions (ncu,
+// 480 k-triangle boxes: 17.6 of 23.5 cycles an instruction, 10.9 of 32 lanes
+// active). Punctual lights are taken vertex-major (VMAJOR: one thread loads
+// its vertex record once and runs every light in order, so the lanes of a
+// warp evaluate the same light) or job-major (one thread per vertex and
+// light: batches that mix scenes of different light counts).
+template <bool VMAJOR, int MINB, bool BATCH>
+__global__ void __launch_bounds__(NEE_THREADS, MINB * 128 / NEE_THREADS) split_nee(const __grid_constant__ WaveArgs a) {
     __shared__ float s_sheen[512];
+    // Punctual lights of a one-scene launch, four 16-byte words each.
+    __shared__ float4 s_light[BATCH || !VMAJOR ? 1 : 4 * NEE_LIGHTS];
     {
         const Scene& s0 = tables_of<BATCH>(a);
         for (uint32_t i = threadIdx.x; i < 512u; i += blockDim.x) s_sheen[i] = tf(s0, s0.P.offs0[1] + i);
+        if (VMAJOR && !BATCH)
+            for (uint32_t i = threadIdx.x; i < 4u * min(a.jobs - 1u, NEE_LIGHTS); i += blockDim.x)
+                s_light[i] = tv4(a.s, a.s.P.offs0[3] + 4u * i);
     }
     __syncthreads();
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
     const uint32_t nv = *((volatile uint32_t*)&a.ctr[4]);
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
-        uint32_t slot = a.q.vslot[v];
+    const uint32_t n_env = *((volatile uint32_t*)&a.ctr[11]), n_area = *((volatile uint32_t*)&a.ctr[12]);
+    Vertex vx;
+    PathCore pc;
+    uint32_t path_seed;
+    ShadowRay sr;
+    for (uint32_t k0 = blockIdx.x * blockDim.x; k0 < n_env; k0 += stride) {
+        __syncthreads();  // see above
+        const uint32_t k = k0 + threadIdx.x;
+        if (k >= n_env) continue;
+        const uint32_t v = a.q.vlight[k], slot = a.q.vslot[v];
         const Scene& s = slot_scene<BATCH>(a, slot);
-        const uint32_t J = BATCH ? min(a.jobs, s.P.cfg[2] + 1u) : a.jobs;  // this scene's NEE jobs
-        Vertex vx;
-        PathCore pc;
-        uint32_t path_seed;
         get_vertex(a, v, &vx, &pc, &path_seed);
-        if (a.st.vis) a.st.vis[slot] = 0u;
-        for (uint32_t j = 0; j < J; j++) {
-            ShadowRay sr;
-            float4 pe = make_float4(0.f, 0.f, 0.f, 0.f);
-            bool queued = nee_job(s, s_sheen, pc, vx, j, &sr);
-            if (queued) {
-                pe = make_float4(sr.pending.x, sr.pending.y, sr.pending.z, 1.0f);
-                uint32_t q = append1(&a.ctr[1]);
-                a.q.sh_o[q] = make_float4(sr.o.x, sr.o.y, sr.o.z, sr.tmax);
-                a.q.sh_d[q] = make_float4(sr.d.x, sr.d.y, sr.d.z, __uint_as_float(sr.skip));
-                a.q.sh_m[q] = make_uint4(slot, j, sr.rid, path_seed);
+        const bool queued = nee_env(s, s_sheen, pc, vx, view_terms(s_sheen, vx.bsdf), &sr);
+        put_job(a, slot, s.P.cfg[2], path_seed, queued, sr);
+    }
+    for (uint32_t k0 = blockIdx.x * blockDim.x; k0 < n_area; k0 += stride) {
+        __syncthreads();  // see above
+        const uint32_t k = k0 + threadIdx.x;
+        if (k >= n_area) continue;
+        const uint32_t v = a.q.vlight[a.vcap - 1u - k], slot = a.q.vslot[v];
+        const Scene& s = slot_scene<BATCH>(a, slot);
+        get_vertex(a, v, &vx, &pc, &path_seed);
+        const bool queued = nee_area(s, s_sheen, pc, vx, view_terms(s_sheen, vx.bsdf), &sr);
+        put_job(a, slot, s.P.cfg[2], path_seed, queued, sr);
+    }
+    if (a.jobs == 1u) return;
+    if (VMAJOR) {
+        for (uint32_t v = first; v < nv; v += stride) {
+            const uint32_t slot = a.q.vslot[v];
+            const Scene& s = slot_scene<BATCH>(a, slot);
+            const uint32_t np = BATCH ? s.P.cfg[2] : a.jobs - 1u;
+            if (BATCH && np == 0u) continue;
+            get_vertex(a, v, &vx, &pc, &path_seed);
+            const ViewTerms vt = view_terms(s_sheen, vx.bsdf);
+#pragma unroll 1
+            for (uint32_t j = 0; j < np; j++) {
+                LightRec rec;
+                if (!BATCH && j < NEE_LIGHTS)
+                    rec = {s_light[4u * j], s_light[4u * j + 1u], s_light[4u * j + 2u], s_light[4u * j + 3u]};
+                else rec = light_rec(s, j);
+                const bool queued = nee_punctual(s, s_sheen, pc, vx, vt, rec, j, &sr);
+                put_job(a, slot, j, path_seed, queued, sr);
             }
-            if (queued || !a.st.vis) a.st.pend[(uint64_t)slot * a.jobs + j] = pe;
+        }
+    } else {
+        const uint64_t total = (uint64_t)nv * (a.jobs - 1u);
+        for (uint64_t t = first; t < total; t += stride) {
+            const uint32_t j = (uint32_t)(t / nv), v = (uint32_t)(t - (uint64_t)j * nv);
+            const uint32_t slot = a.q.vslot[v];
+            const Scene& s = slot_scene<BATCH>(a, slot);
+            if (BATCH && j >= s.P.cfg[2]) continue;  // beyond this scene's punctual lights
+            get_vertex(a, v, &vx, &pc, &path_seed);
+            const bool queued =
+                nee_punctual(s, s_sheen, pc, vx, view_terms(s_sheen, vx.bsdf), light_rec(s, j), j, &sr);
+            put_job(a, slot, j, path_seed, queued, sr);
         }
     }
 }
 
-// Variants: shade kernel for 2 / 3 / 4 resident blocks per SM; the NEE
-// kernel job-major (0-2) or vertex-major (3-5) for 4 / 5 / 6.
+// Variants: shade kernel for at least 4 (0, 1) or 5 resident blocks of 128
+// threads per SM (with registers for 2 or 3 the compiler took up to 178 a
+// thread and the kernel 1.2 to 1.6x the time); the NEE kernel job-major (0-2) or
+// vertex-major (3-5) for 4 / 5 / 6.
 template <bool C, bool B>
 static void* shade_fn(int v) {
-    if (v == 0) return (void*)split_shade<C, 2, B>;
-    if (v == 1) return (void*)split_shade<C, 3, B>;
-    return (void*)split_shade<C, 4, B>;
+    return v < 2 ? (void*)split_shade<C, 5, B> : (void*)split_shade<C, 6, B>;
 }
-template <bool C, bool B>
+template <bool B>
 static void* nee_fn(int v) {
-    if (v == 0) return (void*)split_nee<C, 4, B>;
-    if (v == 1) return (void*)split_nee<C, 5, B>;
-    if (v == 2) return (void*)split_nee<C, 6, B>;
-    if (v == 3) return (void*)split_nee_v<C, 4, B>;
-    if (v == 4) return (void*)split_nee_v<C, 5, B>;
-    return (void*)split_nee_v<C, 6, B>;
+    if (v == 0) return (void*)split_nee<false, 4, B>;
+    if (v == 1) return (void*)split_nee<false, 5, B>;
+    if (v == 2) return (void*)split_nee<false, 6, B>;
+    if (v == 3) return (void*)split_nee<true, 4, B>;
+    if (v == 4) return (void*)split_nee<true, 5, B>;
+    return (void*)split_nee<true, 6, B>;
 }
 
-static cudaError_t persistent(void* fn, const WaveArgs& a, int sms, cudaStream_t st) {
+// One grid of resident blocks, no more than the slots fill.
+static cudaError_t persistent(void* fn, const WaveArgs& a, int sms, cudaStream_t st, unsigned threads) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 128, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, (int)threads, 0);
     WaveArgs copy = a;
     void* args[] = {&copy};
-    return cudaLaunchKernel(fn, dim3((unsigned)(sms * (per_sm > 0 ? per_sm : 1))), dim3(128), args, 0, st);
+    unsigned blocks = (unsigned)(sms * (per_sm > 0 ? per_sm : 1));
+    return cudaLaunchKernel(fn, dim3(std::min(blocks, (a.slots + threads - 1) / threads)), dim3(threads), args, 0, st);
 }
 
 // Batched launches (a.nframes > 0) have no counting build.
 cudaError_t launch_split_logic(const WaveArgs& a, bool count, cudaStream_t st) {
-    unsigned blocks = (a.slots + 127u) / 128u;
+    const unsigned blocks = (a.slots + LOGIC_THREADS - 1u) / LOGIC_THREADS;
     if (a.nframes) {
         if (count) return cudaErrorInvalidValue;
-        split_logic<false, true><<<blocks, 128, 0, st>>>(a);
+        split_logic<false, true><<<blocks, LOGIC_THREADS, 0, st>>>(a);
     } else if (count) {
-        split_logic<true, false><<<blocks, 128, 0, st>>>(a);
+        split_logic<true, false><<<blocks, LOGIC_THREADS, 0, st>>>(a);
     } else {
-        split_logic<false, false><<<blocks, 128, 0, st>>>(a);
+        split_logic<false, false><<<blocks, LOGIC_THREADS, 0, st>>>(a);
     }
     return cudaGetLastError();
 }
 
 cudaError_t launch_split_shade(const WaveArgs& a, bool count, int variant, int sms, cudaStream_t st) {
     variant = variant < 0 ? 0 : (variant > 2 ? 2 : variant);
-    if (a.nframes) return count ? cudaErrorInvalidValue : persistent(shade_fn<false, true>(variant), a, sms, st);
-    return persistent(count ? shade_fn<true, false>(variant) : shade_fn<false, false>(variant), a, sms, st);
+    if (a.nframes) return count ? cudaErrorInvalidValue : persistent(shade_fn<false, true>(variant), a, sms, st, 128);
+    return persistent(count ? shade_fn<true, false>(variant) : shade_fn<false, false>(variant), a, sms, st, 128);
 }
 
 cudaError_t launch_split_nee(const WaveArgs& a, bool count, int variant, int sms, cudaStream_t st) {
     variant = variant < 0 ? 0 : (variant > 5 ? 5 : variant);
-    if (a.nframes) return count ? cudaErrorInvalidValue : persistent(nee_fn<false, true>(variant), a, sms, st);
-    return persistent(count ? nee_fn<true, false>(variant) : nee_fn<false, false>(variant), a, sms, st);
+    if (a.nframes) return count ? cudaErrorInvalidValue : persistent(nee_fn<true>(variant), a, sms, st, NEE_THREADS);
+    return persistent(nee_fn<false>(variant), a, sms, st, NEE_THREADS);
 }
 
 #ifdef OXPT_FAST

@@ -109,6 +109,8 @@ struct WaveQueues {
     // split wavefront (wave_split.cu)
     uint32_t* shade;  // slot ids with a surface hit to shade
     uint32_t* vslot;  // vertex record -> slot
+    uint32_t* vlight;  // vertex records whose last NEE job samples the environment (from the
+                       // front) or an emissive triangle (from the back)
     float4* vrec;     // vertex records, 13 float4 fields, field-major
     // continuation-ray reordering (ray_order.cu): the queue sorted, and per
     // entry its bucket and rank; bucket counts / offsets (2^15)
@@ -129,7 +131,8 @@ struct WaveArgs {
     unsigned long long* work;   // next item
     uint32_t* ctr;              // [0] continuation rays, [1] shadow rays, [2] active slots,
                                 // [3] hits to shade, [4] vertex records, [5] / [6] next
-                                // continuation / shadow ray to walk
+                                // continuation / shadow ray to walk, [11] / [12] vertices
+                                // that sample the environment / an emissive triangle
     uint32_t refill;            // traversal: idle lanes of a warp that take new rays
     float4* out;
     unsigned long long* counters;
