@@ -128,27 +128,28 @@ oxpt_status oxpt_diag_set_l2_window(oxpt_ctx* ctx, int on, uint64_t* granted);
  * at the defaults. Every plan produces bit-identical accumulators; only
  * speed differs.
  *   mode           OXPT_MODE_MEGAKERNEL: one persistent kernel runs whole
- *                  paths; OXPT_MODE_WAVEFRONT: path state in HBM, one
- *                  shading launch and two traversal launches per bounce.
+ *                  paths; OXPT_MODE_WAVEFRONT: path state in HBM, three
+ *                  shading launches (path logic, surface shading, NEE jobs)
+ *                  and two traversal launches per bounce;
+ *                  OXPT_MODE_WAVEFRONT_SPLIT: the same, and fast_shading may
+ *                  be set.
  *   threads, blocks_per_sm, max_paths   megakernel launch shape.
  *   wave_slots     paths in flight (wavefront); wave_items its paths per
  *                  launch round (0 = 2^27: a 1080p frame of 64 spp in one
  *                  round; the result buffer holds 16 bytes per path of a
  *                  round); check_every its bounces between completion
  *                  checks.
- *   shade_variant  wavefront logic kernel compiled for 2 / 3 / 4 resident
- *                  blocks per SM (0 / 1 / 2): registers against occupancy.
+ *   shade_variant  surface shading kernel compiled for 5 (0, 1) or 6 (2)
+ *                  resident blocks per SM: registers against occupancy.
  *   trace_variant  wavefront traversal kernels: 0-2 with local-memory walk
- *                  stacks for 6 / 8 / 10 blocks per SM; 3-5 with short
- *                  stacks in shared memory, alpha tests out of line and
- *                  optional staged top nodes (oxpt_diag_set_walk), for
- *                  6 / 8 / 10 blocks. Default 4.
- *   nee_variant    split wavefront NEE kernel: job-major (0, 1, 2) or
+ *                  stacks for 6 / 8 / 10 blocks per SM; 3-5 on the wide tree
+ *                  (same results) for 6 / 8 / 8 blocks, or, for counting
+ *                  runs, the binary shadow walk and scenes without that
+ *                  tree, with short stacks in shared memory, alpha tests
+ *                  out of line and optional staged top nodes
+ *                  (oxpt_diag_set_walk) for 6 / 8 / 10 blocks. Default 4.
+ *   nee_variant    NEE kernel, punctual lights job-major (0, 1, 2) or
  *                  vertex-major (3, 4, 5) for 4 / 5 / 6 blocks.
- *   OXPT_MODE_WAVEFRONT_SPLIT: the wavefront with the shading of a bounce
- *                  in three kernels (path logic, surface shading, one thread
- *                  per NEE job); shade_variant then applies to the shading
- *                  kernel.
  *   stack          traversal stack entries: 32 or 64; 0 = 32 when the BVH
  *                  is at most 32 levels deep, else 64 (exact either way).
  *   shadow_walk    wavefront shadow rays: 0 = the four-wide tree built on

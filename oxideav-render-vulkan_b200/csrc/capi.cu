@@ -123,7 +123,7 @@ struct oxpt_ctx {
     uint32_t shadow_walk = 0;
     uint32_t closest_walk = 0;  // 1: continuation rays on the four-wide tree (tolerance plan)
     uint32_t fast_shading = 0;  // 1: the split kernels' fast-math build (tolerance plan)
-    // split plan: per-slot visibility masks instead of a pending record per
+    // per-slot visibility masks instead of a pending record per
     // NEE job (oxpt_diag_set_nee_mask; results are the same either way)
     bool nee_mask = true;
     uint32_t shadow_post = 0;  // four-wide shadow walks with postponed leaves (oxpt_diag_set_shadow_postpone)
@@ -370,12 +370,11 @@ uint32_t bvh_depth_of(const uint32_t* geom, uint32_t nodes) {
 oxpt_status ensure_wave(oxpt_ctx* c, uint32_t slots, uint32_t jobs, oxd::WaveState* st, oxd::WaveQueues* q,
                         uint32_t** ctr, unsigned long long** work) {
     size_t P = slots, PJ = (size_t)slots * jobs;
-    bool split = c->mode == OXPT_MODE_WAVEFRONT_SPLIT;
     size_t sizes[] = {P * 8, P * 16, P * 16, P * 16, P * 16, P * 16, P * 16, P * 16, P * 16, P * 4, P * 4,
                       PJ * 16, P * 4, PJ * 16, PJ * 16, PJ * 16, 64,
-                      split ? P * 4 : 0, split ? P * 4 : 0, split ? 13 * P * 16 : 0, P * 4,
-                      (split && jobs <= 32) ? P * 4 : 0, P * 4, PJ * 4, PJ * 4, (size_t)(1u << 17) * 4, PJ * 4,
-                      split ? P * 4 : 0};
+                      P * 4, P * 4, 13 * P * 16, P * 4,
+                      jobs <= 32 ? P * 4 : 0, P * 4, PJ * 4, PJ * 4, (size_t)(1u << 17) * 4, PJ * 4,
+                      P * 4};
     constexpr int NB = 28;
     size_t total = 0;
     for (size_t s : sizes) total += align256(s);
@@ -399,10 +398,10 @@ oxpt_status ensure_wave(oxpt_ctx* c, uint32_t slots, uint32_t jobs, oxd::WaveSta
         ptr[k] = p;
         p += align256(sizes[k]);
     }
-    q->shade = split ? (uint32_t*)ptr[17] : nullptr;
-    q->vslot = split ? (uint32_t*)ptr[18] : nullptr;
-    q->vrec = split ? (float4*)ptr[19] : nullptr;
-    q->vlight = split ? (uint32_t*)ptr[27] : nullptr;
+    q->shade = (uint32_t*)ptr[17];
+    q->vslot = (uint32_t*)ptr[18];
+    q->vrec = (float4*)ptr[19];
+    q->vlight = (uint32_t*)ptr[27];
     st->item = (unsigned long long*)ptr[0];
     st->seed = (uint4*)ptr[1];
     st->beta = (float4*)ptr[2];
@@ -416,7 +415,7 @@ oxpt_status ensure_wave(oxpt_ctx* c, uint32_t slots, uint32_t jobs, oxd::WaveSta
     st->nee_n = (uint32_t*)ptr[10];
     st->pend = (float4*)ptr[11];
     st->frame = (uint32_t*)ptr[20];
-    st->vis = (split && jobs <= 32 && c->nee_mask) ? (uint32_t*)ptr[21] : nullptr;
+    st->vis = (jobs <= 32 && c->nee_mask) ? (uint32_t*)ptr[21] : nullptr;
     q->ext_sorted = (uint32_t*)ptr[22];
     q->ord_key = (uint32_t*)ptr[23];
     q->ord_rank = (uint32_t*)ptr[24];
@@ -496,9 +495,8 @@ cudaError_t wave_init(const oxd::WaveArgs& wa, cudaStream_t st) {
     return e;
 }
 
-// Kernels of one wavefront iteration on `st`: queue reset, shading
-// (one logic kernel, or logic + surface shading + NEE jobs in the split
-// plan), extension and shadow traversal. `wrap(kind, launch)` runs each
+// Kernels of one wavefront iteration on `st`: queue reset, shading (path
+// logic, surface shading, NEE jobs), extension and shadow traversal. `wrap(kind, launch)` runs each
 // launch (timing hooks); returns the kernels enqueued, or -1 on error.
 template <class Wrap>
 int enqueue_iteration(oxpt_ctx* c, const oxd::WaveArgs& wa, const oxd::WaveArgs& wsh, bool count, bool four, int sd,
@@ -514,12 +512,13 @@ int enqueue_iteration(oxpt_ctx* c, const oxd::WaveArgs& wa, const oxd::WaveArgs&
         run(2, [&] { return oxd::fast::launch_split_logic(wa, count, st); });
         run(5, [&] { return oxd::fast::launch_split_shade(wa, count, (int)c->shade_variant, c->sms, st); });
         run(6, [&] { return oxd::fast::launch_split_nee(wa, count, (int)c->nee_variant, c->sms, st); });
-    } else if (c->mode == OXPT_MODE_WAVEFRONT_SPLIT) {
+    } else {
+        // Both wavefront modes: the single shading kernel that mode 1 had was
+        // bound by instruction fetches (20 k-triangle materials, 641 x 359,
+        // 32 spp: 74.6 ms against 12.5 ms for these three).
         run(2, [&] { return oxd::launch_split_logic(wa, count, st); });
         run(5, [&] { return oxd::launch_split_shade(wa, count, (int)c->shade_variant, c->sms, st); });
         run(6, [&] { return oxd::launch_split_nee(wa, count, (int)c->nee_variant, c->sms, st); });
-    } else {
-        run(2, [&] { return oxd::launch_wave_logic(wa, count, (int)c->shade_variant, st); });
     }
     const int sde = (wa.closest4 || (wa.wide && !count && c->trace_variant >= 3)) ? sd4 : sd;
     if (wa.ray_order & 1u) {

@@ -1,20 +1,19 @@
-// Split wavefront: the shading work of a bounce in three small kernels.
+// The shading work of a bounce in three kernels.
 //
-// The single wavefront logic kernel (wavefront.cu) carries texture
-// filtering, the layered BSDF, light sampling and path bookkeeping in one
-// body whose code does not fit the instruction cache. Here a bounce is
+// One kernel with texture filtering, the layered BSDF, light sampling and
+// path bookkeeping in one body does not fit the instruction cache. So:
 //   split_logic  one thread per slot: adds the previous vertex's visible NEE
 //                terms in job order, attenuates in a medium, handles misses
 //                (environment / ambient), finalises finished paths and
 //                regenerates their slots; surface hits go to a shade queue;
 //   split_shade  one thread per queued hit: emission, material, BSDF of the
 //                vertex (written to a vertex record for split_nee), BSDF
-//                sampling and roulette; queues the continuation ray;
-//   split_nee    one thread per (vertex, NEE job), job-major so that a warp
-//                evaluates the same light for 32 vertices;
-// followed by the same extension and shadow traversal kernels. Every path
-// still receives its contributions in the reference's order: the vertex's
-// NEE terms are added by the next split_logic before anything the next
+//                sampling and roulette; queues the continuation ray, and
+//                lists the vertices by the kind of light they sample;
+//   split_nee    the vertices' NEE jobs, one kind of light after the other;
+// followed by the extension and shadow traversal kernels. Every path still
+// receives its contributions in the reference's order: the vertex's NEE
+// terms are added by the next split_logic before anything the next
 // continuation ray finds.
 #include <cooperative_groups.h>
 
@@ -562,10 +561,11 @@ __global__ void __launch_bounds__(NEE_THREADS, MINB * 128 / NEE_THREADS) split_n
     }
 }
 
-// Variants: shade kernel for at least 4 (0, 1) or 5 resident blocks of 128
-// threads per SM (with registers for 2 or 3 the compiler took up to 178 a
-// thread and the kernel 1.2 to 1.6x the time); the NEE kernel job-major (0-2) or
-// vertex-major (3-5) for 4 / 5 / 6.
+// Variants: shade kernel for 5 (0, 1) or 6 blocks of 128 threads per SM (96
+// registers: 3.95 ms of shading per 8 spp of the 1.05 M-triangle frame against
+// 4.3 at 4 blocks; left more registers the compiler took up to 178 and the
+// kernel 5 to 6.9 ms); the NEE kernel job-major (0-2) or vertex-major (3-5)
+// for 4 / 5 / 6 blocks of 128.
 template <bool C, bool B>
 static void* shade_fn(int v) {
     return v < 2 ? (void*)split_shade<C, 5, B> : (void*)split_shade<C, 6, B>;

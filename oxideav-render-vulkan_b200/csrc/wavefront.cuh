@@ -17,13 +17,6 @@ __device__ __forceinline__ uint32_t append(uint32_t* ctr) {
     if (g.thread_rank() == 0) base = atomicAdd(ctr, g.size());
     return g.shfl(base, 0) + g.thread_rank();
 }
-__device__ __forceinline__ unsigned long long fetch_item(unsigned long long* ctr) {
-    namespace cg = cooperative_groups;
-    cg::coalesced_group g = cg::coalesced_threads();
-    unsigned long long base = 0;
-    if (g.thread_rank() == 0) base = atomicAdd(ctr, (unsigned long long)g.size());
-    return g.shfl(base, 0) + g.thread_rank();
-}
 
 constexpr uint32_t WAVE_TRAVERSE_THREADS = 128;
 
@@ -180,12 +173,11 @@ struct WaveArgs {
 cudaError_t launch_order_ext(const WaveArgs& a, int sms, cudaStream_t st);
 cudaError_t launch_order_shadow(const WaveArgs& a, int sms, cudaStream_t st);
 
-// `variant`: 0..2, the occupancy target of the compiled kernel (logic 2 / 3
-// / 4 blocks per SM; traversal 6 / 8 / 10); traversal variants 3..5 run the
-// on-chip-stack kernels of wave_walk.cu (6 / 8 / 10 blocks per SM);
+// Traversal. `variant`: 0..2, the occupancy target of the compiled kernel (6 /
+// 8 / 10 blocks per SM); 3..5 run wide_walk.cu, or wave_walk.cu for counting
+// launches, the binary shadow walk and scenes without a four-wide tree;
 // `stack`: 32 or 64 entries.
 // With a.nframes > 0 the batched kernels run (count must then be false).
-cudaError_t launch_wave_logic(const WaveArgs& a, bool count, int variant, cudaStream_t st);
 cudaError_t launch_wave_extend(const WaveArgs& a, bool count, int variant, int stack, int sms, cudaStream_t st);
 // four: any-hit walk over the four-wide tree (Scene::bvh4) instead of the
 // binary one; stack: 32 or 64 entries, enough for the tree walked.
