@@ -354,7 +354,8 @@ unsigned blocks(uint32_t n, unsigned t) { return (n + t - 1) / t; }
     } while (0)
 
 Collapse collapse4_device(const uint32_t* w, uint32_t nodes, cudaStream_t st, uint32_t** out, size_t* out_cap, uint32_t* n4,
-                          uint32_t* root_ref, uint32_t* need, std::string* err, size_t more_per_node, size_t more) {
+                          uint32_t* root_ref, uint32_t* need, std::string* err, size_t more_per_node, size_t more,
+                          Arena* mem) {
     using namespace bvh4b;
     *n4 = 0;
     *need = 1;
@@ -369,6 +370,9 @@ Collapse collapse4_device(const uint32_t* w, uint32_t nodes, cudaStream_t st, ui
     std::vector<uint32_t> level_start;
     uint32_t h[2] = {0, 0};
     const uint32_t cap = nodes / 2 + 1;
+    auto scratch = [&](auto** p, size_t bytes) {
+        return mem ? mem->get(p, bytes) : cudaMallocAsync((void**)p, bytes, st);
+    };
     if (cudaMemcpyAsync(root_words, w, 32, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess) {
         *err = "four-wide tree: root readback";
@@ -381,11 +385,11 @@ Collapse collapse4_device(const uint32_t* w, uint32_t nodes, cudaStream_t st, ui
         return Collapse::BUILT;
     }
     *root_ref = 0;
-    CK4(cudaMallocAsync((void**)&items, (size_t)cap * sizeof(Item), st));
-    CK4(cudaMallocAsync((void**)&counts, (size_t)cap * 4, st));
-    CK4(cudaMallocAsync((void**)&sums, (size_t)blocks(cap, 1024) * 4, st));
-    CK4(cudaMallocAsync((void**)&sums2, 1024 * 4, st));
-    CK4(cudaMallocAsync((void**)&ctr, 8, st));  // total, bad
+    CK4(scratch(&items, (size_t)cap * sizeof(Item)));
+    CK4(scratch(&counts, (size_t)cap * 4));
+    CK4(scratch(&sums, (size_t)blocks(cap, 1024) * 4));
+    CK4(scratch(&sums2, 1024 * 4));
+    CK4(scratch(&ctr, 8));  // total, bad
     {
         Item root{};
         root.b = 0;
@@ -436,7 +440,7 @@ Collapse collapse4_device(const uint32_t* w, uint32_t nodes, cudaStream_t st, ui
     CK4(cudaGetLastError());
     {
         const size_t bytes = (size_t)*n4 * (128 + more_per_node) + more + 4;
-        if (!*out || *out_cap < bytes) {  // the caller's buffer, when it is large enough
+        if (!*out || *out_cap < bytes || *out_cap / 2 > bytes) {  // the caller's buffer, when it fits
             if (*out) cudaFree(*out);
             *out = nullptr;
             *out_cap = 0;
@@ -455,7 +459,7 @@ Collapse collapse4_device(const uint32_t* w, uint32_t nodes, cudaStream_t st, ui
     *need = h[0];
 done:
     for (void* p : {(void*)items, (void*)counts, (void*)sums, (void*)sums2, (void*)ctr})
-        if (p) cudaFreeAsync(p, st);
+        if (p && !mem) cudaFreeAsync(p, st);
     if (res != Collapse::BUILT) {
         cudaStreamSynchronize(st);
         *n4 = 0;

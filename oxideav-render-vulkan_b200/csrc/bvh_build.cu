@@ -25,6 +25,8 @@
 #include <string>
 #include <vector>
 
+#include "scene_prep.cuh"
+
 #include "../../include/oxpt_diag.h"
 #include "../host/bvh_gpu.hpp"
 
@@ -915,8 +917,16 @@ namespace bvhb {
         }                                                                \
     } while (0)
 
-bool build_on_device(const float* pos, uint32_t n, cudaStream_t st, uint32_t** words_out, uint32_t** slots_out,
-                     uint32_t* nodes_out, uint32_t* depth_out, uint32_t* launches_out, std::string* err) {
+size_t scratch_bytes(uint32_t n) {
+    const size_t m = n, huge = m / HUGE_N + 2;
+    return m * (3 * 16 + 2 * 4 + 64 + 2 * sizeof(Job) + sizeof(Decision) + 4 + 4) + (m / 1024 + 1) * 4 +
+           (m / LARGE + 2) * 4 + huge * (4 + sizeof(HugeNode) + sizeof(HugeAcc)) + (m / CHUNK + huge + 1) * 4 + 4096 +
+           20 * 256;  // the pieces' alignment
+}
+
+bool build_on_device(const float* pos, uint32_t n, cudaStream_t st, Arena* mem, uint32_t** words_out,
+                     uint32_t** slots_out, uint32_t* nodes_out, uint32_t* depth_out, uint32_t* launches_out,
+                     std::string* err) {
     *words_out = *slots_out = nullptr;
     *nodes_out = *depth_out = 0;
     if (launches_out) *launches_out = 0;
@@ -940,26 +950,26 @@ bool build_on_device(const float* pos, uint32_t n, cudaStream_t st, uint32_t** w
     const size_t max_large = n / LARGE + 2, max_huge = n / HUGE_N + 2, max_chunks = n / CHUNK + max_huge + 1;
     uint32_t K = 1, nodes = 1, levels = 0, launches = 0;
     uint32_t M = 0, Lg = 0, H = 0;  // this level's medium / large / huge nodes
-    BK(cudaMallocAsync((void**)&blo, (size_t)n * 16, st));
-    BK(cudaMallocAsync((void**)&bhi, (size_t)n * 16, st));
-    BK(cudaMallocAsync((void**)&cen, (size_t)n * 16, st));
-    BK(cudaMallocAsync((void**)&ids, (size_t)n * 4, st));
-    BK(cudaMallocAsync((void**)&ids2, (size_t)n * 4, st));
-    BK(cudaMallocAsync((void**)&words, max_nodes * 32, st));
-    BK(cudaMallocAsync((void**)&jobs, max_jobs * sizeof(Job), st));
-    BK(cudaMallocAsync((void**)&next, max_jobs * sizeof(Job), st));
-    BK(cudaMallocAsync((void**)&dec, max_jobs * sizeof(Decision), st));
-    BK(cudaMallocAsync((void**)&excl, max_jobs * 4, st));
-    BK(cudaMallocAsync((void**)&sums, ((max_jobs + 1023) / 1024) * 4, st));
-    BK(cudaMallocAsync((void**)&sums2, 1024 * 4, st));
-    BK(cudaMallocAsync((void**)&ctr, 4 * 4, st));
-    BK(cudaMallocAsync((void**)&l_medium, max_jobs * 4, st));
-    BK(cudaMallocAsync((void**)&l_large, max_large * 4, st));
-    BK(cudaMallocAsync((void**)&l_huge, max_huge * 4, st));
-    BK(cudaMallocAsync((void**)&hn, max_huge * sizeof(HugeNode), st));
-    BK(cudaMallocAsync((void**)&acc, max_huge * sizeof(HugeAcc), st));
-    BK(cudaMallocAsync((void**)&chunk_left, max_chunks * 4, st));
-    BK(cudaMallocAsync((void**)&total_chunks, 4, st));
+    BK(mem->get(&blo, (size_t)n * 16));
+    BK(mem->get(&bhi, (size_t)n * 16));
+    BK(mem->get(&cen, (size_t)n * 16));
+    BK(mem->get(&ids, (size_t)n * 4));
+    BK(mem->get(&ids2, (size_t)n * 4));
+    BK(mem->get(&words, max_nodes * 32));
+    BK(mem->get(&jobs, max_jobs * sizeof(Job)));
+    BK(mem->get(&next, max_jobs * sizeof(Job)));
+    BK(mem->get(&dec, max_jobs * sizeof(Decision)));
+    BK(mem->get(&excl, max_jobs * 4));
+    BK(mem->get(&sums, ((max_jobs + 1023) / 1024) * 4));
+    BK(mem->get(&sums2, 1024 * 4));
+    BK(mem->get(&ctr, 4 * 4));
+    BK(mem->get(&l_medium, max_jobs * 4));
+    BK(mem->get(&l_large, max_large * 4));
+    BK(mem->get(&l_huge, max_huge * 4));
+    BK(mem->get(&hn, max_huge * sizeof(HugeNode)));
+    BK(mem->get(&acc, max_huge * sizeof(HugeAcc)));
+    BK(mem->get(&chunk_left, max_chunks * 4));
+    BK(mem->get(&total_chunks, 4));
     tri_prep<<<(n + 255) / 256, 256, 0, st>>>(pos, n, blo, bhi, cen, ids);
     BK(cudaGetLastError());
     launches++;
@@ -1031,15 +1041,10 @@ bool build_on_device(const float* pos, uint32_t n, cudaStream_t st, uint32_t** w
     }
     *words_out = words;
     *slots_out = ids;
-    words = ids = nullptr;
     *nodes_out = nodes;
     *depth_out = levels;
     if (launches_out) *launches_out = launches;
 done:
-    void* ptrs[] = {blo, bhi, cen, ids, ids2, words, excl, sums, sums2, ctr, jobs, next, dec,
-                    l_medium, l_large, l_huge, hn, acc, chunk_left, total_chunks};
-    for (void* p : ptrs)
-        if (p) cudaFreeAsync(p, st);  // stream-ordered: no device-wide synchronisation
     if (!ok) cudaStreamSynchronize(st);
     return ok;
 }
@@ -1057,11 +1062,13 @@ bool build_bvh_device(int device, const std::vector<float>& tri_pos, BvhBuild* o
     float* pos = nullptr;
     uint32_t *words = nullptr, *slots = nullptr, nodes = 0, depth = 0;
     cudaStream_t st = nullptr;
+    oxd::Arena mem;
     BK(cudaSetDevice(device));
+    BK(mem.begin(oxd::bvhb::scratch_bytes(n)));
     BK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     BK(cudaMalloc((void**)&pos, tri_pos.size() * 4));
     BK(cudaMemcpyAsync(pos, tri_pos.data(), tri_pos.size() * 4, cudaMemcpyHostToDevice, st));
-    if (!oxd::bvhb::build_on_device(pos, n, st, &words, &slots, &nodes, &depth, nullptr, err)) {
+    if (!oxd::bvhb::build_on_device(pos, n, st, &mem, &words, &slots, &nodes, &depth, nullptr, err)) {
         ok = false;
         goto done;
     }
@@ -1074,8 +1081,6 @@ bool build_bvh_device(int device, const std::vector<float>& tri_pos, BvhBuild* o
 done:
     if (st) cudaStreamSynchronize(st);
     if (pos) cudaFree(pos);
-    if (words) cudaFreeAsync(words, st);
-    if (slots) cudaFreeAsync(slots, st);
     if (st) {
         cudaStreamSynchronize(st);
         cudaStreamDestroy(st);

@@ -158,6 +158,7 @@ struct oxpt_ctx {
     std::vector<uint64_t> bgraph_alt_key;
     uint64_t graph_builds = 0;
     unsigned long long* dev_tally = nullptr;  // graph loops: kernels launched, iterations
+    oxd::Arena build_mem;  // scratch of oxpt_build_scene
     float build_ms[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // last oxpt_build_scene: phases, wall, tree, launches
     size_t geom_cap = 0, attrs_cap = 0, atlas_cap = 0;  // bytes of the owned scene buffers
     size_t bvh4_cap = 0, tables_cap = 0;
@@ -786,14 +787,14 @@ static oxpt_status build_wide(oxpt_ctx* c, const float4* geom, uint32_t nodes, s
 // The four-wide tree of the scene now in c->geom, collapsed on the device
 // (the host collapse's words); a tree too wide or deep for the device pass
 // is read back and collapsed on the host.
-static oxpt_status device_bvh4(oxpt_ctx* c) {
+static oxpt_status device_bvh4(oxpt_ctx* c, oxd::Arena* mem = nullptr) {
     c->bvh4_built = false;
     uint32_t* out = reinterpret_cast<uint32_t*>(c->bvh4);  // reused when large enough
     uint32_t n4 = 0, root = 0xffffffffu, need = 1;
     std::string e;
     const uint32_t* words = reinterpret_cast<const uint32_t*>(c->geom);
     oxd::Collapse r = oxd::collapse4_device(words, c->node_count, c->stream, &out, &c->bvh4_cap, &n4, &root, &need, &e,
-                                            WIDE_NODE_BYTES, c->slot_count * 4);
+                                            WIDE_NODE_BYTES, c->slot_count * 4, mem);
     c->bvh4 = reinterpret_cast<float4*>(out);
     if (r == oxd::Collapse::FAILED) return fail(c, OXPT_E_CUDA, e);
     if (r == oxd::Collapse::REFUSED) return OXPT_OK;  // the binary walk serves every ray
@@ -933,36 +934,57 @@ oxpt_status oxpt_build_scene(oxpt_ctx* c, const oxpt_scene_src* src, uint32_t* l
     if (oxpt_status sa = activate_staged(c)) return sa;
     oxpt_status s = set_device(c);
     if (s) return s;
-    CK(c, cudaStreamSynchronize(c->stream), "sync before scene build");
+    // The new scene is written over the old one's buffers where they fit, so
+    // every stream that may still read those (views, batches) is waited for,
+    // as freeing them would.
+    CK(c, cudaDeviceSynchronize(), "sync before scene build");
     c->has_scene = false;
     drop_borrowed_scene(c);
-    // The old scene's buffers go first: the build needs the room.
-    realloc_dev(c, &c->geom, 0, "geom buffer");
-    realloc_dev(c, &c->attrs, 0, "attribute buffer");
-    realloc_dev(c, &c->atlas, 0, "texture atlas");
-    c->geom_cap = c->attrs_cap = c->atlas_cap = 0;
-    realloc_dev(c, &c->bvh4, 0, "four-wide tree");
-    c->bvh4_cap = 0;
     c->bvh4_built = false;
     auto t0 = std::chrono::steady_clock::now();
     oxd::prep::DeviceScene ds;
     std::string e;
-    if ((s = oxd::prep::build_scene(*src, c->stream, &ds, light_slots, &e))) return fail(c, s, e);
+    for (int attempt = 0;; attempt++) {
+        ds.geom = c->geom;
+        ds.geom_cap = c->geom_cap;
+        ds.attrs = c->attrs;
+        ds.attrs_cap = c->attrs_cap;
+        ds.atlas = c->atlas;
+        ds.atlas_cap = c->atlas_cap;
+        s = oxd::prep::build_scene(*src, c->stream, &c->build_mem, &ds, light_slots, &e);
+        c->geom = ds.geom;
+        c->geom_cap = ds.geom_cap;
+        c->attrs = ds.attrs;
+        c->attrs_cap = ds.attrs_cap;
+        c->atlas = ds.atlas;
+        c->atlas_cap = ds.atlas_cap;
+        if (s != OXPT_E_NOMEM || attempt) break;
+        // Short of memory: the old scene's buffers go first.
+        realloc_dev(c, &c->geom, 0, "geom buffer");
+        realloc_dev(c, &c->attrs, 0, "attribute buffer");
+        realloc_dev(c, &c->atlas, 0, "texture atlas");
+        realloc_dev(c, &c->bvh4, 0, "four-wide tree");
+        c->geom_cap = c->attrs_cap = c->atlas_cap = c->bvh4_cap = 0;
+        c->build_mem.end();
+    }
+    if (s) {
+        c->build_mem.end();
+        return fail(c, s, e);
+    }
     auto t1 = std::chrono::steady_clock::now();
-    c->geom = ds.geom;
     c->geom_vec4 = ds.geom_vec4;
-    c->geom_cap = ds.geom_vec4 * 16;
-    c->attrs_cap = ds.slot_count * 192;
-    c->atlas_cap = (size_t)src->atlas_side * src->atlas_side * src->atlas_layers * 8;
-    c->attrs = ds.attrs;
     c->slot_count = ds.slot_count;
-    c->atlas = ds.atlas;
     c->side = src->atlas_side;
     c->layers = src->atlas_layers;
     c->node_count = ds.node_count;
     c->bvh_depth = std::min(ds.depth, 65u);  // bvh_depth_of's cap
     if (c->stack == 32 && c->bvh_depth > 32) c->stack = 0;
-    if ((s = device_bvh4(c))) return s;
+    c->build_mem.rewind(0);  // the build's pieces: it waited for its streams
+    s = device_bvh4(c, &c->build_mem);
+    if (!s && c->build_mem.bytes() > oxd::Arena::KEEP)
+        CK(c, cudaStreamSynchronize(c->stream), "scene build");  // the block goes back
+    c->build_mem.end();
+    if (s) return s;
     auto t2 = std::chrono::steady_clock::now();
     for (int k = 0; k < 4; k++) c->build_ms[k] = ds.phase_ms[k];
     c->build_ms[4] = std::chrono::duration<float, std::milli>(t2 - t0).count();
@@ -1533,7 +1555,7 @@ oxpt_status oxpt_ctx_memory(const oxpt_ctx* c, uint64_t out[4]) {
     out[1] = (c->borrowed_tables ? 0 : (uint64_t)c->table_words * 4) + c->back.tables_cap;
     uint64_t px = (uint64_t)c->w * c->h;
     out[2] = c->accum ? px * 16 + (c->img8 ? px * 4 : 0) + (c->img32 ? px * 16 : 0) : 0;
-    out[3] = c->out_cap * 16 + c->wave_bytes + c->batch_cap * sizeof(oxd::BatchFrame);
+    out[3] = c->out_cap * 16 + c->wave_bytes + c->batch_cap * sizeof(oxd::BatchFrame) + c->build_mem.bytes();
     return OXPT_OK;
 }
 

@@ -457,9 +457,25 @@ void atlas_work(AtlasJob* j) {
 
 }  // namespace
 
-oxpt_status build_scene(const oxpt_scene_src& src, cudaStream_t st, DeviceScene* out, uint32_t* light_slots,
-                        std::string* err) {
-    *out = DeviceScene{};
+namespace {
+
+// Keeps a buffer that holds `bytes` and is at most twice that.
+template <class T>
+cudaError_t reserve(T** p, size_t* cap, size_t bytes) {
+    if (*p && bytes && *cap >= bytes && *cap / 2 <= bytes) return cudaSuccess;
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+    *cap = 0;
+    cudaError_t e = cudaMalloc((void**)p, bytes);
+    if (e == cudaSuccess) *cap = bytes;
+    else *p = nullptr;
+    return e;
+}
+
+}  // namespace
+
+oxpt_status build_scene(const oxpt_scene_src& src, cudaStream_t st, Arena* mem, DeviceScene* out,
+                        uint32_t* light_slots, std::string* err) {
     uint64_t ntri64 = 0, stream_floats = 0;
     oxpt_status status = check_src(src, light_slots, &ntri64, &stream_floats, err);
     if (status) return status;
@@ -469,7 +485,7 @@ oxpt_status build_scene(const oxpt_scene_src& src, cudaStream_t st, DeviceScene*
     MeshRec* recs = nullptr;
     uint32_t *bases = nullptr, *light_of = nullptr, *lights = nullptr, *lslots = nullptr;
     uint32_t *words = nullptr, *slots = nullptr;
-    DeviceScene ds;
+    DeviceScene& ds = *out;  // the caller owns its buffers whatever the outcome
     Stager stage(st);
     cudaError_t e = cudaSuccess;
     std::vector<MeshRec> hrec;
@@ -479,7 +495,8 @@ oxpt_status build_scene(const oxpt_scene_src& src, cudaStream_t st, DeviceScene*
     AtlasJob job;
     std::thread worker;
     bool working = false;
-    uint32_t bvh_launches = 0;
+    uint32_t bvh_launches = 0, non_empty = 0;
+    const size_t atlas_bytes = (size_t)src.atlas_side * src.atlas_side * src.atlas_layers * 8;
 
 #define PK(expr, what)                                            \
     do {                                                          \
@@ -501,30 +518,39 @@ oxpt_status build_scene(const oxpt_scene_src& src, cudaStream_t st, DeviceScene*
         level_dims(ch.width, ch.height, 1, &w1, &h1);
         max_lvl1 = std::max<uint64_t>(max_lvl1, (uint64_t)w1 * h1);
     }
-    PK(cudaMalloc((void**)&ds.atlas, (size_t)src.atlas_side * src.atlas_side * src.atlas_layers * 8), "texture atlas");
+    for (uint32_t i = 0; i < src.n_meshes; i++) non_empty += src.meshes[i].ntri ? 1 : 0;
+    // One block for everything that does not outlive the build.
+    PK(mem->begin((max_tex + 2 * max_lvl1) * 16 + (size_t)n * (36 + 4) + stream_floats * 4 +
+                  (size_t)src.n_lights * 8 + (size_t)non_empty * (sizeof(MeshRec) + 4) + 16 * 256 +
+                  bvhb::scratch_bytes(n)),
+       "scratch");
+    PK(reserve(&ds.atlas, &ds.atlas_cap, atlas_bytes), "texture atlas");
+    PK(reserve(&ds.attrs, &ds.attrs_cap, (size_t)n * 12 * 16), "attribute buffer");
     job.atlas = ds.atlas;
     if (src.n_chains) {
-        PK(cudaMalloc((void**)&job.tex, max_tex * 16), "texture staging");
-        PK(cudaMalloc((void**)&job.lvl_a, max_lvl1 * 16), "mip level");
-        PK(cudaMalloc((void**)&job.lvl_b, max_lvl1 * 16), "mip level");
+        PK(mem->get(&job.tex, max_tex * 16), "texture staging");
+        PK(mem->get(&job.lvl_a, max_lvl1 * 16), "mip level");
+        PK(mem->get(&job.lvl_b, max_lvl1 * 16), "mip level");
+        PK(cudaStreamCreateWithFlags(&job.st, cudaStreamNonBlocking), "texture stream");
     }
-    PK(cudaStreamCreateWithFlags(&job.st, cudaStreamNonBlocking), "texture stream");
     PK(cudaEventCreate(&job.begin), "timing events");
     PK(cudaEventCreate(&job.end), "timing events");
     // Device buffers of the geometry half.
-    PK(cudaMalloc((void**)&pos, (size_t)n * 36), "positions");
-    PK(cudaMalloc((void**)&streams, std::max<uint64_t>(stream_floats, 1) * 4), "attribute streams");
-    PK(cudaMalloc((void**)&light_of, (size_t)n * 4), "light lookup");
-    PK(cudaMalloc((void**)&lslots, std::max(src.n_lights, 1u) * 4), "light slots");
-    if (src.n_lights) PK(cudaMalloc((void**)&lights, (size_t)src.n_lights * 4), "light list");
+    PK(mem->get(&pos, (size_t)n * 36), "positions");
+    PK(mem->get(&streams, std::max<uint64_t>(stream_floats, 1) * 4), "attribute streams");
+    PK(mem->get(&light_of, (size_t)n * 4), "light lookup");
+    PK(mem->get(&lslots, std::max(src.n_lights, 1u) * 4), "light slots");
+    if (src.n_lights) PK(mem->get(&lights, (size_t)src.n_lights * 4), "light list");
     {
-        uint32_t non_empty = 0;
-        for (uint32_t i = 0; i < src.n_meshes; i++) non_empty += src.meshes[i].ntri ? 1 : 0;
-        PK(cudaMalloc((void**)&recs, (size_t)non_empty * sizeof(MeshRec)), "mesh records");
-        PK(cudaMalloc((void**)&bases, (size_t)non_empty * 4), "mesh bases");
+        PK(mem->get(&recs, (size_t)non_empty * sizeof(MeshRec)), "mesh records");
+        PK(mem->get(&bases, (size_t)non_empty * 4), "mesh bases");
     }
-    worker = std::thread(atlas_work, &job);
-    working = true;
+    if (src.n_chains) {
+        worker = std::thread(atlas_work, &job);
+        working = true;
+    } else {  // an atlas without textures is zeros
+        PK(cudaMemsetAsync(ds.atlas, 0, atlas_bytes, st), "texture atlas");
+    }
 
     PK(stage.init(), "pinned staging");
     PK(cudaEventRecord(ev[0], st), "timing");
@@ -567,15 +593,14 @@ oxpt_status build_scene(const oxpt_scene_src& src, cudaStream_t st, DeviceScene*
     }
     PK(cudaEventRecord(ev[1], st), "timing");
     // BVH (syncs the stream once per level).
-    if (!bvhb::build_on_device(pos, n, st, &words, &slots, &ds.node_count, &ds.depth, &bvh_launches, err)) {
+    if (!bvhb::build_on_device(pos, n, st, mem, &words, &slots, &ds.node_count, &ds.depth, &bvh_launches, err)) {
         status = err->find("out of memory") != std::string::npos ? OXPT_E_NOMEM : OXPT_E_CUDA;
         goto fail_status;
     }
     PK(cudaEventRecord(ev[2], st), "timing");
     ds.slot_count = n;
     ds.geom_vec4 = (size_t)ds.node_count * 2 + (size_t)n * 3;
-    PK(cudaMalloc((void**)&ds.geom, ds.geom_vec4 * 16), "geom buffer");
-    PK(cudaMalloc((void**)&ds.attrs, (size_t)n * 12 * 16), "attribute buffer");
+    PK(reserve(&ds.geom, &ds.geom_cap, ds.geom_vec4 * 16), "geom buffer");
     PK(cudaMemcpyAsync(ds.geom, words, (size_t)ds.node_count * 32, cudaMemcpyDeviceToDevice, st), "node copy");
     emit_slots<<<grid_of((size_t)n * 15, 256), 256, 0, st>>>(n, slots, pos, streams, recs, bases, (uint32_t)hrec.size(),
                                                               light_of, (uint4*)(ds.geom + (size_t)ds.node_count * 2),
@@ -590,7 +615,7 @@ oxpt_status build_scene(const oxpt_scene_src& src, cudaStream_t st, DeviceScene*
     if (src.n_lights)
         PK(cudaMemcpyAsync(light_slots, lslots, (size_t)src.n_lights * 4, cudaMemcpyDeviceToHost, st), "light slots");
     PK(cudaStreamSynchronize(st), "scene build");
-    worker.join();
+    if (working) worker.join();
     working = false;
     if (job.e != cudaSuccess) {
         e = job.e;
@@ -600,23 +625,15 @@ oxpt_status build_scene(const oxpt_scene_src& src, cudaStream_t st, DeviceScene*
     cudaEventElapsedTime(&ds.phase_ms[0], ev[0], ev[1]);
     cudaEventElapsedTime(&ds.phase_ms[1], ev[1], ev[2]);
     cudaEventElapsedTime(&ds.phase_ms[2], ev[2], ev[3]);
-    if (cudaEventElapsedTime(&ds.phase_ms[3], job.begin, job.end) != cudaSuccess) ds.phase_ms[3] = 0.0f;
+    if (!src.n_chains || cudaEventElapsedTime(&ds.phase_ms[3], job.begin, job.end) != cudaSuccess) ds.phase_ms[3] = 0.0f;
     // the BVH's, flattening (+ two for lights), mip levels
     ds.launches = bvh_launches + 1 + (src.n_lights ? 2 : 0) + job.launches;
     (void)cudaGetLastError();
-    cudaFreeAsync(words, st);
-    cudaFreeAsync(slots, st);
-    {
-        void* temps[] = {pos, streams, job.tex, job.lvl_a, job.lvl_b, recs, bases, light_of, lights, lslots};
-        for (void* p : temps)
-            if (p) cudaFree(p);
-    }
     for (auto x : ev) cudaEventDestroy(x);
     cudaEventDestroy(job.begin);
     cudaEventDestroy(job.end);
-    cudaStreamDestroy(job.st);
+    if (job.st) cudaStreamDestroy(job.st);
     stage.release();
-    *out = std::move(ds);
     return OXPT_OK;
 #undef PK
 
@@ -628,15 +645,6 @@ fail_status:
     cudaStreamSynchronize(st);
     if (job.st) cudaStreamSynchronize(job.st);
     stage.release();
-    if (words) cudaFreeAsync(words, st);
-    if (slots) cudaFreeAsync(slots, st);
-    cudaStreamSynchronize(st);
-    {
-        void* temps[] = {pos, streams, job.tex, job.lvl_a, job.lvl_b, recs, bases, light_of, lights, lslots,
-                         ds.geom, ds.attrs, ds.atlas};
-        for (void* p : temps)
-            if (p) cudaFree(p);
-    }
     for (auto x : ev)
         if (x) cudaEventDestroy(x);
     if (job.begin) cudaEventDestroy(job.begin);

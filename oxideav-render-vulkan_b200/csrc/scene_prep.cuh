@@ -10,16 +10,81 @@
 #include "../../include/oxpt.h"
 
 namespace oxd {
+
+// Scratch memory of a scene build: pieces of one block, handed out in order
+// and given back all at once. A build used to make some 35 allocations, each
+// of which can cost a page-table update (a 4800-triangle sync took 4 to 24 ms,
+// most of it there). A request beyond the block is allocated by itself.
+// Everything handed out is used on the build's stream, or on the atlas stream
+// that the build waits for, before release().
+class Arena {
+  public:
+    // Blocks up to this size stay for the next build of the same owner.
+    static constexpr size_t KEEP = 64u << 20;
+    ~Arena() { drop(); }
+    // Starts a build that needs about `bytes`.
+    cudaError_t begin(size_t bytes) {
+        release();
+        if (bytes <= cap_) return cudaSuccess;
+        drop();
+        cudaError_t e = cudaMalloc((void**)&base_, bytes);
+        if (e != cudaSuccess) base_ = nullptr;
+        else cap_ = bytes;
+        return e;
+    }
+    template <class T>
+    cudaError_t get(T** p, size_t bytes) {
+        const size_t at = (used_ + 255) & ~(size_t)255;
+        if (at + bytes <= cap_) {
+            *p = reinterpret_cast<T*>(base_ + at);
+            used_ = at + bytes;
+            return cudaSuccess;
+        }
+        void* own = nullptr;
+        cudaError_t e = cudaMalloc(&own, bytes ? bytes : 1);
+        *p = static_cast<T*>(own);
+        if (e == cudaSuccess) more_.push_back(own);
+        return e;
+    }
+    // Pieces handed out since `mark` are free again (a caller's piece
+    // outside the block stays until release).
+    size_t mark() const { return used_; }
+    void rewind(size_t mark) { used_ = mark; }
+    void release() {
+        used_ = 0;
+        for (void* p : more_) cudaFree(p);
+        more_.clear();
+    }
+    // The end of a build.
+    void end() {
+        release();
+        if (cap_ > KEEP) drop();
+    }
+    size_t bytes() const { return cap_; }
+    Arena() = default;
+    Arena(const Arena&) = delete;
+    Arena& operator=(const Arena&) = delete;
+
+  private:
+    void drop() {
+        release();
+        if (base_) cudaFree(base_);
+        base_ = nullptr;
+        cap_ = 0;
+    }
+    char* base_ = nullptr;
+    size_t cap_ = 0, used_ = 0;
+    std::vector<void*> more_;
+};
 namespace bvhb {
 
 // Binned-SAH BVH over n triangles whose positions (9 floats each) are in
 // device memory, built on stream st. On success *words (nodes x 8 words)
-// and *slots (leaf slot -> triangle, n entries) are stream-ordered device
-// allocations (cudaMallocAsync on st) that the caller frees with
-// cudaFreeAsync. Scratch is stream-ordered too, so the build never waits
-// for other streams' work. False with *err when an allocation or launch
-// fails.
-bool build_on_device(const float* pos, uint32_t n, cudaStream_t st, uint32_t** words, uint32_t** slots,
+// and *slots (leaf slot -> triangle, n entries) are pieces of `mem`, as all
+// scratch is (scratch_bytes(n) in all). False with *err when an allocation
+// or launch fails.
+size_t scratch_bytes(uint32_t n);
+bool build_on_device(const float* pos, uint32_t n, cudaStream_t st, Arena* mem, uint32_t** words, uint32_t** slots,
                      uint32_t* nodes, uint32_t* depth, uint32_t* launches, std::string* err);
 
 }  // namespace bvhb
@@ -31,12 +96,13 @@ bool build_on_device(const float* pos, uint32_t n, cudaStream_t st, uint32_t** w
 // it; untouched when the root is a leaf; with room for more_per_node bytes a
 // node and `more` behind the nodes), *root_ref and *need are set. REFUSED: the host collapse
 // refuses the tree too (keep the binary walk). UNSUPPORTED: deeper than
-// 64 four-wide levels (collapse on the host). FAILED: a CUDA error.
+// 64 four-wide levels (collapse on the host). FAILED: a CUDA error. Scratch
+// comes from `mem`, or is stream-ordered (cudaMallocAsync) without it.
 enum class Collapse { BUILT, REFUSED, UNSUPPORTED, FAILED };
 Collapse collapse4_device(const uint32_t* words, uint32_t nodes, cudaStream_t st, uint32_t** out, size_t* out_cap,
                           uint32_t* n4,
                           uint32_t* root_ref, uint32_t* need, std::string* err, size_t more_per_node = 0,
-                          size_t more = 0);
+                          size_t more = 0, Arena* mem = nullptr);
 // Levels of the binary tree (65 when deeper than 64 or malformed), as the
 // host's depth walk counts them.
 bool binary_depth_device(const uint32_t* words, uint32_t nodes, cudaStream_t st, uint32_t* depth, std::string* err);
@@ -49,13 +115,16 @@ cudaError_t launch_leaf_map(const uint32_t* words, uint32_t nodes, uint32_t* map
 
 namespace prep {
 
-// Device buffers of one prepared scene, owned by the caller afterwards.
+// Device buffers of one prepared scene, owned by the caller before and
+// afterwards: a build writes into those it is given when they are large
+// enough (and not more than twice too large) and replaces the others.
 struct DeviceScene {
     float4* geom = nullptr;   // nodes, then triangles in leaf-slot order
-    size_t geom_vec4 = 0;
+    size_t geom_vec4 = 0, geom_cap = 0;
     float4* attrs = nullptr;  // 12 float4 per slot
-    size_t slot_count = 0;
+    size_t slot_count = 0, attrs_cap = 0;
     uint2* atlas = nullptr;   // side x side x layers RGBA16F texels
+    size_t atlas_cap = 0;
     uint32_t node_count = 0, depth = 0;
 
     // Device time of the phases (CUDA events): source upload, BVH, slot
@@ -64,10 +133,11 @@ struct DeviceScene {
     uint32_t launches = 0;  // kernels this build launched
 };
 
-// Builds every buffer of `src` on st (oxpt_build_scene). On failure nothing
-// stays allocated and *err says why.
-oxpt_status build_scene(const oxpt_scene_src& src, cudaStream_t st, DeviceScene* out, uint32_t* light_slots,
-                        std::string* err);
+// Builds every buffer of `src` on st (oxpt_build_scene), with scratch from
+// `mem`. Nothing may still read the buffers given in *out. On failure *out
+// holds whatever buffers exist, without a scene in them, and *err says why.
+oxpt_status build_scene(const oxpt_scene_src& src, cudaStream_t st, Arena* mem, DeviceScene* out,
+                        uint32_t* light_slots, std::string* err);
 
 }  // namespace prep
 }  // namespace oxd
