@@ -183,6 +183,33 @@ __device__ __forceinline__ float4 pattern(const uint32_t* dirs, const Sampler& s
     pattern_u(dirs, s, p, u);
     return {to_unit(u[0]), to_unit(u[1]), to_unit(u[2]), to_unit(u[3])};
 }
+// The same points from a table of 8 x 16 entries in shared memory: entry
+// 16 n + v is the exclusive or of the four dimensions' direction numbers of
+// the bits set in v << 4 n. Eight loads for a point instead of a loop over
+// the set bits (16 of a scrambled index) per dimension.
+__device__ __forceinline__ void sobol_nibbles(const uint32_t* dirs, uint4* nib) {
+    for (uint32_t e = threadIdx.x; e < 128u; e += blockDim.x) {
+        uint32_t r[4] = {0u, 0u, 0u, 0u};
+        for (uint32_t b = 0; b < 4u; b++)
+            if ((e >> b) & 1u)
+                for (uint32_t d = 0; d < 4u; d++) r[d] ^= dirs[d * 32u + 4u * (e >> 4) + b];
+        nib[e] = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+}
+__device__ __forceinline__ float4 pattern(const uint4* nib, const Sampler& s, uint32_t p) {
+    const uint32_t seed = hash_mix(s.pixel_seed, p), i = nus(s.index, seed);
+    uint4 r = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (uint32_t n = 0; n < 8u; n++) {
+        const uint4 t = nib[16u * n + ((i >> (4u * n)) & 15u)];
+        r.x ^= t.x;
+        r.y ^= t.y;
+        r.z ^= t.z;
+        r.w ^= t.w;
+    }
+    return {to_unit(nus(r.x, hash_mix(seed, 0u))), to_unit(nus(r.y, hash_mix(seed, 1u))),
+            to_unit(nus(r.z, hash_mix(seed, 2u))), to_unit(nus(r.w, hash_mix(seed, 3u)))};
+}
 __device__ __forceinline__ float coin(const Sampler& s, uint32_t ray, uint32_t tri) {
     return to_unit(hash_mix(hash_mix(s.path_seed, ray), tri));
 }

@@ -45,7 +45,8 @@ struct ShadowRay {
 
 // Camera ray (pathtrace.wgsl:1715-1732). Returns the ray origin; the
 // direction is pc->d.
-__device__ __forceinline__ f3 start_path(const Scene& s, const uint32_t* sobol, uint32_t x, uint32_t y,
+template <class Sobol>  // the direction numbers, or their table (sobol_nibbles)
+__device__ __forceinline__ f3 start_path(const Scene& s, const Sobol* sobol, uint32_t x, uint32_t y,
                                          uint32_t index, Sampler* smp, PathCore* pc) {
     *smp = make_sampler(s.P.dims[2], x, y, index);
     float4 p0 = pattern(sobol, *smp, 0u);
@@ -106,8 +107,8 @@ __device__ __forceinline__ int after_ray(const Scene& s, PathCore& pc, bool got,
 // The rest of the PATH branch at a surface hit (pathtrace.wgsl:1799-1861):
 // emission with MIS, unlit, the bounce limit and the vertex's BSDF.
 // PATH_VERTEX: *v holds the vertex and NEE / BSDF sampling follow.
-template <bool COUNT>
-__device__ __forceinline__ int shade_hit(const Scene& s, const float* sheen, const uint32_t* sobol,
+template <bool COUNT, class Sobol>
+__device__ __forceinline__ int shade_hit(const Scene& s, const float* sheen, const Sobol* sobol,
                                          const Sampler& smp, PathCore& pc, const Hit& hit, uint32_t hmat,
                                          Vertex* v, unsigned long long* shaded) {
     const uint32_t strategy = s.P.cfg[1];
@@ -308,7 +309,8 @@ __device__ __forceinline__ bool nee_job(const Scene& s, const float* sheen, cons
 // BSDF sampling, medium transition and roulette (pathtrace.wgsl:1999-2039).
 // False when the path ends; otherwise pc.d is the new direction, pc.k the
 // new bounce and the new ray origin is returned through *origin.
-__device__ __forceinline__ bool continue_path(const Scene& s, const float* sheen, const uint32_t* sobol,
+template <class Sobol>
+__device__ __forceinline__ bool continue_path(const Scene& s, const float* sheen, const Sobol* sobol,
                                               const Sampler& smp, PathCore& pc, const Vertex& v, f3* origin) {
     float4 pb_u = pattern(sobol, smp, 1u + 2u * pc.k);
     BSample bs = bsdf_sample(sheen, v.bsdf, pb_u.x, pb_u.y, pb_u.z);

@@ -256,7 +256,7 @@ __device__ __forceinline__ uint32_t logic_slot(const WaveArgs& a, uint32_t i) {
 // Starts the path of launch item `item` in slot i.
 template <bool BATCH>
 __device__ __forceinline__ void start_slot(const WaveArgs& a, uint32_t i, unsigned long long item,
-                                           const uint32_t* s_sobol) {
+                                           const uint4* s_sobol) {
     PathCore pc;
     Sampler smp;
     uint32_t f = BATCH ? frame_of1(a, item) : 0u;
@@ -287,7 +287,8 @@ constexpr uint32_t LOGIC_THREADS = 256u;
 template <bool COUNT, bool BATCH>
 __global__ void __launch_bounds__(LOGIC_THREADS, 4) split_logic(const __grid_constant__ WaveArgs a) {
     constexpr uint32_t WARPS = LOGIC_THREADS / 32u;
-    __shared__ uint32_t s_sobol[128];
+    __shared__ uint32_t s_dirs[128];
+    __shared__ uint4 s_sobol[128];
     __shared__ uint32_t s_surface[WARPS], s_free[WARPS];
     __shared__ uint32_t s_shade_at, s_ext_at;
     __shared__ unsigned long long s_item_at;
@@ -326,9 +327,13 @@ __global__ void __launch_bounds__(LOGIC_THREADS, 4) split_logic(const __grid_con
     }
     if (frees) {
         const Scene& s0 = tables_of<BATCH>(a);
-        for (uint32_t k = threadIdx.x; k < 128u; k += LOGIC_THREADS) s_sobol[k] = tw(s0, s0.P.offs0[0] + k);
+        for (uint32_t k = threadIdx.x; k < 128u; k += LOGIC_THREADS) s_dirs[k] = tw(s0, s0.P.offs0[0] + k);
     }
     __syncthreads();
+    if (frees) {  // the same for the whole block
+        sobol_nibbles(s_dirs, s_sobol);
+        __syncthreads();
+    }
     if (surface) a.q.shade[s_shade_at + my_surface] = i;
     if (!free_slot) return;
     const unsigned long long item = s_item_at + my_free;
@@ -342,14 +347,16 @@ __global__ void __launch_bounds__(LOGIC_THREADS, 4) split_logic(const __grid_con
 
 template <bool COUNT, int MINB, bool BATCH>
 __global__ void __launch_bounds__(128, MINB) split_shade(const __grid_constant__ WaveArgs a) {
-    __shared__ uint32_t s_sobol[128];
+    __shared__ uint32_t s_dirs[128];
+    __shared__ uint4 s_sobol[128];
     __shared__ float s_sheen[512];
     {
         const Scene& s0 = tables_of<BATCH>(a);
-        for (uint32_t i = threadIdx.x; i < 128u; i += blockDim.x) s_sobol[i] = tw(s0, s0.P.offs0[0] + i);
+        for (uint32_t i = threadIdx.x; i < 128u; i += blockDim.x) s_dirs[i] = tw(s0, s0.P.offs0[0] + i);
         for (uint32_t i = threadIdx.x; i < 512u; i += blockDim.x) s_sheen[i] = tf(s0, s0.P.offs0[1] + i);
     }
     __syncthreads();
+    sobol_nibbles(s_dirs, s_sobol);  // read after the loop's barrier
     const uint32_t n = *((volatile uint32_t*)&a.ctr[3]);
     unsigned long long shaded = 0;
     for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < n; q0 += gridDim.x * blockDim.x) {
