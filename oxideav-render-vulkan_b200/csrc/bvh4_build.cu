@@ -281,8 +281,9 @@ __global__ void depth_level(const uint32_t* frontier, uint32_t K, const uint32_t
 // then per child the inner node's index or the leaf's reference. Inner
 // children come first, so that child k of them is node (word 12) + k. The
 // low four bits of the x step say which children are inner nodes, those of
-// the y step which are leaves. Boxes are rounded outwards by at least 1/64
-// of a step (more than the walk's arithmetic loses on the bytes).
+// the y step which are leaves. The corner is that of byte value -32768, since
+// the walk reads a byte q as the float 32768 + q. Boxes are rounded outwards
+// by at least 1/32 of a step (more than the walk's arithmetic loses on them).
 __global__ void wide_nodes(const uint4* bvh4, uint32_t n4, uint32_t* out) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n4) return;
@@ -309,11 +310,13 @@ __global__ void wide_nodes(const uint4* bvh4, uint32_t n4, uint32_t* out) {
         float step = fmaxf((mx - mn) * (1.0f / 253.0f), fmaxf(fmaxf(fabsf(mn), fabsf(mx)) * 1.0e-7f, 1.0e-30f));
         const uint32_t mask = ax == 0 ? (1u << inner) - 1u : (ax == 1 ? (1u << kids) - (1u << inner) : 0u);
         step = __uint_as_float((__float_as_uint(step) & ~15u) | mask);
-        const float corner = mn - step * 0.5f;
+        // The stored corner is where the byte plane of value -32768 lies.
+        const float corner = (float)((double)mn - 32768.5 * (double)step);
+        const double zero = (double)corner + 32768.0 * (double)step;
         uint32_t ql = 0, qh = 0;
         for (int j = 0; j < kids; j++) {
-            const uint32_t a = (uint32_t)fminf(fmaxf(floorf((lo[from[j]] - corner) / step - 0.015625f), 0.0f), 255.0f);
-            const uint32_t b = (uint32_t)fminf(fmaxf(ceilf((hi[from[j]] - corner) / step + 0.015625f), 0.0f), 255.0f);
+            const uint32_t a = (uint32_t)fminf(fmaxf(floorf((float)(((double)lo[from[j]] - zero) / step) - 0.03125f), 0.0f), 255.0f);
+            const uint32_t b = (uint32_t)fminf(fmaxf(ceilf((float)(((double)hi[from[j]] - zero) / step) + 0.03125f), 0.0f), 255.0f);
             ql |= a << (8 * j);
             qh |= b << (8 * j);
         }

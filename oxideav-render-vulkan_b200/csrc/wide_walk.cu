@@ -15,9 +15,12 @@
 // * Leaves that pass are noted in the lane's column; when FLUSH are noted (or
 //   no lane has node work) the warp tests one (ray, triangle) pair per lane:
 //   full warps whatever the rays' mix of nodes and leaves is.
-// A 64-spp 1080p frame of that scene: closest hits 89.9 -> 42 ms, shadow rays
-// 135.9 -> 71 ms (17 -> 24 active lanes in a node step; now bound by issue:
-// about 77% of cycles issue). FLUSH of 24 to 48, 4 to 10 entries in shared
+// * A node step is about 190 instructions: the stored corner lets one fused
+//   operation place a plane, an any-hit walk takes its next node straight from
+//   the group of waiting siblings (nearest first gained it nothing).
+// A 64-spp 1080p frame of that scene: closest hits 89.9 -> 41 ms, shadow rays
+// 135.9 -> 67 ms (24 active lanes in a node step; now bound by issue: about 77%
+// of cycles issue). FLUSH of 24 to 48, 4 to 10 entries in shared
 // memory, 2 to 8 steps between checks and 12 pending leaves were within 3%
 // of each other or worse; 48 registers a thread (10 blocks) spilled and were
 // 1.2 to 1.9x slower than 64.
@@ -27,8 +30,8 @@
 // * Boxes are widened by eta = 2^-18 x the largest coordinate of the scene
 //   box and the ray origin. With u = 2^-24 the watertight test places the
 //   hit point within 46 u of that coordinate from the ray, and what the
-//   slab arithmetic below loses is within 6 u of it and within 1/128 of a
-//   byte step (the bytes leave 1/64), so a triangle that passes the
+//   slab arithmetic below loses is within 8 u of it and within 1/128
+//   of a byte step (the bytes leave 1/32), so a triangle that passes the
 //   triangle test at distance t has t between the widened entry and exit
 //   distances of every box around it: with a distance limit T, all triangles
 //   with t <= T are tested, in whatever order the boxes come.
@@ -109,10 +112,11 @@ __device__ __forceinline__ u8x ld32(const void* p) {
     return r;
 }
 
-// What a node step needs of a ray: reciprocal direction, origin moved back by
-// eta along it, and what that adds to a far plane's distance.
+// What a node step needs of a ray: reciprocal direction, the product of it
+// with the origin moved along it by eta, negated, and what moving the origin
+// back by eta instead adds to a far plane's distance.
 struct NodeRay {
-    float inv[3], on[3], c[3];
+    float inv[3], nb[3], c[3];
 };
 
 __device__ __forceinline__ NodeRay node_ray(const Scene& s, const Ray& r) {
@@ -126,7 +130,7 @@ __device__ __forceinline__ NodeRay node_ray(const Scene& s, const Ray& r) {
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         n.inv[a] = iv[a];
-        n.on[a] = iv[a] < 0.0f ? oo[a] - eta : oo[a] + eta;
+        n.nb[a] = -((iv[a] < 0.0f ? oo[a] - eta : oo[a] + eta) * iv[a]);
         n.c[a] = fabsf(2.0f * eta * iv[a]);
     }
     return n;
@@ -383,7 +387,8 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
                         }
                         tl = o.w;
                         sp = group = 0u;
-                        guard = 4u * s.bvh4_nodes + 8u;
+                        if (!EXT) group = s.bvh4_root << 4 | 1u;
+                        guard = 4u * STEPS * min(s.bvh4_nodes, 1u << 27) + 64u;
                         cur = s.bvh4_root;
                         if (cur & LEAF_BIT) {  // a tree of one leaf
                             M.leaf[0][lane] = cur;
@@ -400,14 +405,23 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
             }
             drained = __any_sync(FULL, drained || none_left);
         }
-        // Node steps.
+        // Node steps. A tree's nodes are visited at most once each.
+        if (guard < (uint32_t)STEPS) {
+            if (cur != NONE) atomicOr(a.err, 1u);
+            cur = NONE;
+        } else {
+            guard -= STEPS;
+        }
 #pragma unroll 1
         for (int step = 0; step < STEPS; step++) {
             if (cur == NONE || leaves > LEAFCAP - 4u) continue;
-            if (guard-- == 0u) {
-                atomicOr(a.err, 1u);
-                cur = NONE;
-                continue;
+            if (!EXT) {
+                if (!(group & 15u)) {
+                    sp--;
+                    group = sp < SS ? M.stack[sp][lane] : deep[sp];
+                }
+                cur = (group >> 4) + (uint32_t)__ffs(group & 15u) - 1u;
+                group &= group - 1u;
             }
             const char* nd = nodes + (uint64_t)cur * 64u;
             const u8x v0 = ld32(nd), v1 = ld32(nd + 32);
@@ -415,7 +429,7 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
 #pragma unroll
             for (int ax = 0; ax < 3; ax++) {
                 const float A = __uint_as_float(v0.v[3 + ax]) * nr.inv[ax];
-                const float bn = __fmaf_rn(-32768.0f, A, (__uint_as_float(v0.v[ax]) - nr.on[ax]) * nr.inv[ax]);
+                const float bn = __fmaf_rn(__uint_as_float(v0.v[ax]), nr.inv[ax], nr.nb[ax]);
                 const float bf = bn + nr.c[ax];
                 const uint32_t lo = ax < 2 ? v0.v[6 + ax] : v1.v[0], hi = v1.v[1 + ax];
                 const bool neg = nr.inv[ax] < 0.0f;
@@ -437,6 +451,18 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
 #pragma unroll
             for (int k = 0; k < 4; k++)
                 if (leaf & (1u << k)) M.leaf[leaves++][lane] = v1.v[4 + k];
+            if (!EXT) {
+                if (inner) {
+                    if (group & 15u) {
+                        if (sp < SS) M.stack[sp][lane] = group;
+                        else deep[sp] = group;
+                        sp++;
+                    }
+                    group = v1.v[4] << 4 | inner;
+                }
+                if (!(group & 15u) && sp == 0u) cur = NONE;
+                continue;
+            }
             if (inner) {
                 // The nearest inner child is next, its siblings wait as a group.
                 uint32_t key[4];
