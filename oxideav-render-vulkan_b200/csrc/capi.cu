@@ -1731,7 +1731,24 @@ oxpt_status batch_graph_run(oxpt_ctx* e, const std::vector<oxd::WaveArgs>& args,
         const oxd::WaveArgs& a0 = args[0];
         key.insert(key.end(), {(uint64_t)(uintptr_t)a0.s.geom, a0.s.geom_vec4, a0.s.P.env[3], a0.one_scene,
                                a0.closest4, a0.wide, a0.walk_lim, a0.walk_stage, (uint64_t)(uintptr_t)a0.st.vis,
-                               a0.shadow_post, a0.ray_order, a0.l2_share, a0.l2_max_window});
+                               a0.shadow_post, a0.ray_order, a0.l2_share, a0.l2_max_window, a0.one_frame});
+        if (a0.one_frame) {
+            // The scene in the kernels' arguments; the camera and the seed come
+            // from the frame record.
+            const oxd::Scene& sc = a0.s;
+            const oxpt_params& P = sc.P;
+            key.insert(key.end(), {(uint64_t)(uintptr_t)sc.attrs, sc.slot_count, (uint64_t)(uintptr_t)sc.tables,
+                                   sc.table_words, (uint64_t)(uintptr_t)sc.atlas, sc.side, sc.layers,
+                                   (uint64_t)(uintptr_t)sc.bvh4, sc.bvh4_root, sc.bvh4_nodes, sc.bvh4_ok,
+                                   (uint64_t)(uintptr_t)sc.wide, (uint64_t)(uintptr_t)sc.leaf_of, P.dims[0],
+                                   P.dims[1], P.dims[3]});
+            for (const uint32_t* v : {P.cfg, P.env, P.offs0, P.offs1, P.offs2}) key.insert(key.end(), v, v + 4);
+            for (float f : P.fparams) {
+                uint32_t u;
+                std::memcpy(&u, &f, 4);
+                key.push_back(u);
+            }
+        }
     }
     for (size_t k = 0; k < rounds.size(); k++) {
         const oxd::WaveArgs& wa = args[k];
@@ -1980,6 +1997,7 @@ oxpt_status oxpt_refine_batch(oxpt_ctx* e, const oxpt_batch_frame* fr, uint32_t 
         if (s0 && one) {
             base.s = scene_view(s0);
             base.one_scene = 1u;
+            base.one_frame = n == 1 ? 1u : 0u;
         }
     }
     if ((s = ensure_wave(e, pmax, J, &base.st, &base.q, &base.ctr, &base.work))) {

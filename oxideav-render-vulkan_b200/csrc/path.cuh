@@ -107,8 +107,9 @@ __device__ __forceinline__ int after_ray(const Scene& s, PathCore& pc, bool got,
 // The rest of the PATH branch at a surface hit (pathtrace.wgsl:1799-1861):
 // emission with MIS, unlit, the bounce limit and the vertex's BSDF.
 // PATH_VERTEX: *v holds the vertex and NEE / BSDF sampling follow.
+// `cam` holds the camera (a scene's own view of it may be older).
 template <bool COUNT, class Sobol>
-__device__ __forceinline__ int shade_hit(const Scene& s, const float* sheen, const Sobol* sobol,
+__device__ __forceinline__ int shade_hit(const Scene& s, const Scene& cam, const float* sheen, const Sobol* sobol,
                                          const Sampler& smp, PathCore& pc, const Hit& hit, uint32_t hmat,
                                          Vertex* v, unsigned long long* shaded) {
     const uint32_t strategy = s.P.cfg[1];
@@ -118,7 +119,7 @@ __device__ __forceinline__ int shade_hit(const Scene& s, const float* sheen, con
     bool double_sided = (mflags & 4u) != 0u;
     Lod lod = base_lod();
     if (pc.k == 0u) {
-        float cw = s.P.eye[3] > 0.5f ? s.P.up[3] : s.P.up[3] * hit.t;
+        float cw = cam.P.eye[3] > 0.5f ? cam.P.up[3] : cam.P.up[3] * hit.t;
         lod = {cw, pc.d};
     }
     bool flip = !hit.front && double_sided;
@@ -168,7 +169,7 @@ __device__ __forceinline__ int on_path_hit(const Scene& s, const float* sheen, c
                                            uint32_t hmat, Vertex* v, unsigned long long* shaded) {
     int r = after_ray(s, pc, got, hit);
     if (r != PATH_SURFACE) return r;
-    return shade_hit<COUNT>(s, sheen, sobol, smp, pc, hit, hmat, v, shaded);
+    return shade_hit<COUNT>(s, s, sheen, sobol, smp, pc, hit, hmat, v, shaded);
 }
 
 // Whether a light in direction `to` (any length) certainly adds nothing at

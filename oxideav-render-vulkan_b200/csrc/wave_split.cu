@@ -151,16 +151,23 @@ __device__ __forceinline__ uint32_t frame_of1(const WaveArgs& a, unsigned long l
     return lo;
 }
 
-template <bool BATCH>
+// What a launch traces: one scene's frame given in its arguments; frames of a
+// batch, whose records are in memory; or a batch of one frame, whose scene is
+// in the arguments all the same (constant memory; read from a record, every
+// field is a load of its own) and whose camera, seed and sample range come
+// from the record, so that a captured graph serves the next step.
+enum Launch : int { PLAIN = 0, FRAMES = 1, ONE_FRAME = 2 };
+
+template <int M>
 __device__ __forceinline__ const Scene& slot_scene(const WaveArgs& a, uint32_t i) {
-    return BATCH ? a.frames[a.st.frame[i]].s : a.s;
+    return M == FRAMES ? a.frames[a.st.frame[i]].s : a.s;
 }
 
 // Shared-memory tables come from the first frame in a batched launch (the
 // host checks that every scene holds the same words).
-template <bool BATCH>
+template <int M>
 __device__ __forceinline__ const Scene& tables_of(const WaveArgs& a) {
-    return BATCH ? a.frames[0].s : a.s;
+    return M == FRAMES ? a.frames[0].s : a.s;
 }
 
 // Radiance-cache inputs of a vertex: position normalised to the scene's
@@ -201,7 +208,7 @@ enum LogicOutcome : uint32_t { SLOT_SURFACE, SLOT_FREED, SLOT_EMPTY };
 // Adds the slot's NEE terms and takes its path past its ray: a surface hit to
 // shade, or a finished path, whose result is stored. What every slot reads is
 // loaded first, together.
-template <bool BATCH>
+template <int M>
 __device__ __forceinline__ uint32_t logic_slot(const WaveArgs& a, uint32_t i) {
     const uint32_t J = a.jobs;
     PathCore pc;
@@ -240,7 +247,7 @@ __device__ __forceinline__ uint32_t logic_slot(const WaveArgs& a, uint32_t i) {
             if (pc.in_medium) pc.sigma = xyz(a.st.sigma[i]);
             Hit hit;
             hit.t = __uint_as_float(h.y);
-            r = after_ray(slot_scene<BATCH>(a, i), pc, h.x != NONE, hit);
+            r = after_ray(slot_scene<M>(a, i), pc, h.x != NONE, hit);
             if (r == PATH_SURFACE) a.st.beta[i] = make_float4(pc.beta.x, pc.beta.y, pc.beta.z, pc.prev_pdf);
         }
     }
@@ -254,22 +261,23 @@ __device__ __forceinline__ uint32_t logic_slot(const WaveArgs& a, uint32_t i) {
 }
 
 // Starts the path of launch item `item` in slot i.
-template <bool BATCH>
+template <int M>
 __device__ __forceinline__ void start_slot(const WaveArgs& a, uint32_t i, unsigned long long item,
                                            const uint4* s_sobol) {
     PathCore pc;
     Sampler smp;
-    uint32_t f = BATCH ? frame_of1(a, item) : 0u;
-    const Scene& s = BATCH ? a.frames[f].s : a.s;
-    unsigned long long local = BATCH ? item - a.frames[f].base : item;
-    uint32_t npix = BATCH ? a.frames[f].npix : a.npix;
-    uint32_t y0 = BATCH ? a.frames[f].y0 : a.y0, first = BATCH ? a.frames[f].first : a.first;
+    constexpr bool REC = M != PLAIN;
+    uint32_t f = M == FRAMES ? frame_of1(a, item) : 0u;
+    const Scene& s = REC ? a.frames[f].s : a.s;
+    unsigned long long local = REC ? item - a.frames[f].base : item;
+    uint32_t npix = REC ? a.frames[f].npix : a.npix;
+    uint32_t y0 = REC ? a.frames[f].y0 : a.y0, first = REC ? a.frames[f].first : a.first;
     uint32_t it = (uint32_t)(local / npix);
     uint32_t q = (uint32_t)(local - (unsigned long long)it * npix);
     uint32_t yy = q / s.P.dims[0];
     f3 o = start_path(s, s_sobol, q - yy * s.P.dims[0], y0 + yy, first + it, &smp, &pc);
     a.st.item[i] = item;
-    if (BATCH) a.st.frame[i] = f;
+    if (M == FRAMES) a.st.frame[i] = f;
     if (a.nrc.on) {
         a.nrc.s_tidx[i] = NONE;
         a.nrc.s_tail[i] = NONE;
@@ -284,7 +292,7 @@ constexpr uint32_t LOGIC_THREADS = 256u;
 // items once. Each warp asking for itself made five atomics a warp on one
 // 64-byte line the kernel's bound (4.2 M slots: 365 us whether it moved 1.3
 // or 0.6 GB).
-template <bool COUNT, bool BATCH>
+template <bool COUNT, int M>
 __global__ void __launch_bounds__(LOGIC_THREADS, 4) split_logic(const __grid_constant__ WaveArgs a) {
     constexpr uint32_t WARPS = LOGIC_THREADS / 32u;
     __shared__ uint32_t s_dirs[128];
@@ -294,7 +302,7 @@ __global__ void __launch_bounds__(LOGIC_THREADS, 4) split_logic(const __grid_con
     __shared__ unsigned long long s_item_at;
     const uint32_t i = blockIdx.x * LOGIC_THREADS + threadIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (i == 0u) a.ctr[11] = a.ctr[12] = 0u;  // counted by split_shade
-    const uint32_t out = i < a.slots ? logic_slot<BATCH>(a, i) : (uint32_t)SLOT_EMPTY;
+    const uint32_t out = i < a.slots ? logic_slot<M>(a, i) : (uint32_t)SLOT_EMPTY;
     const bool surface = out == SLOT_SURFACE, free_slot = !surface && i < a.slots;
     const unsigned below = (1u << lane) - 1u;
     const unsigned ms = __ballot_sync(0xffffffffu, surface), mf = __ballot_sync(0xffffffffu, free_slot);
@@ -326,7 +334,7 @@ __global__ void __launch_bounds__(LOGIC_THREADS, 4) split_logic(const __grid_con
         if (COUNT && starts) atomicAdd(a.counters + C_PATHS, (unsigned long long)starts);
     }
     if (frees) {
-        const Scene& s0 = tables_of<BATCH>(a);
+        const Scene& s0 = tables_of<M>(a);
         for (uint32_t k = threadIdx.x; k < 128u; k += LOGIC_THREADS) s_dirs[k] = tw(s0, s0.P.offs0[0] + k);
     }
     __syncthreads();
@@ -338,20 +346,20 @@ __global__ void __launch_bounds__(LOGIC_THREADS, 4) split_logic(const __grid_con
     if (!free_slot) return;
     const unsigned long long item = s_item_at + my_free;
     if (item < a.total) {
-        start_slot<BATCH>(a, i, item, s_sobol);
+        start_slot<M>(a, i, item, s_sobol);
         a.q.ext[s_ext_at + my_free] = i;
     } else if (out != SLOT_EMPTY) {
         a.st.rad[i].w = __uint_as_float(ST_EMPTY);
     }
 }
 
-template <bool COUNT, int MINB, bool BATCH>
+template <bool COUNT, int MINB, int M>
 __global__ void __launch_bounds__(128, MINB) split_shade(const __grid_constant__ WaveArgs a) {
     __shared__ uint32_t s_dirs[128];
     __shared__ uint4 s_sobol[128];
     __shared__ float s_sheen[512];
     {
-        const Scene& s0 = tables_of<BATCH>(a);
+        const Scene& s0 = tables_of<M>(a);
         for (uint32_t i = threadIdx.x; i < 128u; i += blockDim.x) s_dirs[i] = tw(s0, s0.P.offs0[0] + i);
         for (uint32_t i = threadIdx.x; i < 512u; i += blockDim.x) s_sheen[i] = tf(s0, s0.P.offs0[1] + i);
     }
@@ -364,14 +372,14 @@ __global__ void __launch_bounds__(128, MINB) split_shade(const __grid_constant__
         uint32_t q = q0 + threadIdx.x;
         if (q >= n) continue;
         uint32_t i = a.q.shade[q];
-        const Scene& s = slot_scene<BATCH>(a, i);
+        const Scene& s = slot_scene<M>(a, i);
         PathCore pc;
         Sampler smp;
         load_state(a, i, &pc, &smp);
         uint32_t hmat;
         Hit hit = load_hit(a, i, &hmat);
         Vertex vx;
-        int r = shade_hit<COUNT>(s, s_sheen, s_sobol, smp, pc, hit, hmat, &vx, &shaded);
+        int r = shade_hit<COUNT>(s, M == ONE_FRAME ? a.frames[0].s : s, s_sheen, s_sobol, smp, pc, hit, hmat, &vx, &shaded);
         if (r != PATH_VERTEX) {
             save_rad(a, i, pc, ST_ENDING);
             continue;
@@ -445,7 +453,7 @@ __global__ void __launch_bounds__(128, MINB) split_shade(const __grid_constant__
         uint32_t v = append1(&a.ctr[4]);
         put_vertex(a, v, vx, pc, smp.path_seed);
         a.q.vslot[v] = i;
-        const uint32_t jobs = BATCH ? s.P.cfg[2] + 1u : a.jobs;
+        const uint32_t jobs = M == FRAMES ? s.P.cfg[2] + 1u : a.jobs;
         a.st.nee_n[i] = jobs;
         if (a.st.vis) a.st.vis[i] = 0u;
         const uint32_t kind = sampled_light(s, vx.pl_u.z);
@@ -494,13 +502,14 @@ __device__ __forceinline__ void put_job(const WaveArgs& a, uint32_t slot, uint32
 // its vertex record once and runs every light in order, so the lanes of a
 // warp evaluate the same light) or job-major (one thread per vertex and
 // light: batches that mix scenes of different light counts).
-template <bool VMAJOR, int MINB, bool BATCH>
+template <bool VMAJOR, int MINB, int M>
 __global__ void __launch_bounds__(NEE_THREADS, MINB * 128 / NEE_THREADS) split_nee(const __grid_constant__ WaveArgs a) {
+    constexpr bool BATCH = M == FRAMES;
     __shared__ float s_sheen[512];
     // Punctual lights of a one-scene launch, four 16-byte words each.
     __shared__ float4 s_light[BATCH || !VMAJOR ? 1 : 4 * NEE_LIGHTS];
     {
-        const Scene& s0 = tables_of<BATCH>(a);
+        const Scene& s0 = tables_of<M>(a);
         for (uint32_t i = threadIdx.x; i < 512u; i += blockDim.x) s_sheen[i] = tf(s0, s0.P.offs0[1] + i);
         if (VMAJOR && !BATCH)
             for (uint32_t i = threadIdx.x; i < 4u * min(a.jobs - 1u, NEE_LIGHTS); i += blockDim.x)
@@ -519,7 +528,7 @@ __global__ void __launch_bounds__(NEE_THREADS, MINB * 128 / NEE_THREADS) split_n
         const uint32_t k = k0 + threadIdx.x;
         if (k >= n_env) continue;
         const uint32_t v = a.q.vlight[k], slot = a.q.vslot[v];
-        const Scene& s = slot_scene<BATCH>(a, slot);
+        const Scene& s = slot_scene<M>(a, slot);
         get_vertex(a, v, &vx, &pc, &path_seed);
         const bool queued = nee_env(s, s_sheen, pc, vx, view_terms(s_sheen, vx.bsdf), &sr);
         put_job(a, slot, s.P.cfg[2], path_seed, queued, sr);
@@ -529,7 +538,7 @@ __global__ void __launch_bounds__(NEE_THREADS, MINB * 128 / NEE_THREADS) split_n
         const uint32_t k = k0 + threadIdx.x;
         if (k >= n_area) continue;
         const uint32_t v = a.q.vlight[a.vcap - 1u - k], slot = a.q.vslot[v];
-        const Scene& s = slot_scene<BATCH>(a, slot);
+        const Scene& s = slot_scene<M>(a, slot);
         get_vertex(a, v, &vx, &pc, &path_seed);
         const bool queued = nee_area(s, s_sheen, pc, vx, view_terms(s_sheen, vx.bsdf), &sr);
         put_job(a, slot, s.P.cfg[2], path_seed, queued, sr);
@@ -538,7 +547,7 @@ __global__ void __launch_bounds__(NEE_THREADS, MINB * 128 / NEE_THREADS) split_n
     if (VMAJOR) {
         for (uint32_t v = first; v < nv; v += stride) {
             const uint32_t slot = a.q.vslot[v];
-            const Scene& s = slot_scene<BATCH>(a, slot);
+            const Scene& s = slot_scene<M>(a, slot);
             const uint32_t np = BATCH ? s.P.cfg[2] : a.jobs - 1u;
             if (BATCH && np == 0u) continue;
             get_vertex(a, v, &vx, &pc, &path_seed);
@@ -558,7 +567,7 @@ __global__ void __launch_bounds__(NEE_THREADS, MINB * 128 / NEE_THREADS) split_n
         for (uint64_t t = first; t < total; t += stride) {
             const uint32_t j = (uint32_t)(t / nv), v = (uint32_t)(t - (uint64_t)j * nv);
             const uint32_t slot = a.q.vslot[v];
-            const Scene& s = slot_scene<BATCH>(a, slot);
+            const Scene& s = slot_scene<M>(a, slot);
             if (BATCH && j >= s.P.cfg[2]) continue;  // beyond this scene's punctual lights
             get_vertex(a, v, &vx, &pc, &path_seed);
             const bool queued =
@@ -573,18 +582,18 @@ __global__ void __launch_bounds__(NEE_THREADS, MINB * 128 / NEE_THREADS) split_n
 // 4.3 at 4 blocks; left more registers the compiler took up to 178 and the
 // kernel 5 to 6.9 ms); the NEE kernel job-major (0-2) or vertex-major (3-5)
 // for 4 / 5 / 6 blocks of 128.
-template <bool C, bool B>
+template <bool C, int M>
 static void* shade_fn(int v) {
-    return v < 2 ? (void*)split_shade<C, 5, B> : (void*)split_shade<C, 6, B>;
+    return v < 2 ? (void*)split_shade<C, 5, M> : (void*)split_shade<C, 6, M>;
 }
-template <bool B>
+template <int M>
 static void* nee_fn(int v) {
-    if (v == 0) return (void*)split_nee<false, 4, B>;
-    if (v == 1) return (void*)split_nee<false, 5, B>;
-    if (v == 2) return (void*)split_nee<false, 6, B>;
-    if (v == 3) return (void*)split_nee<true, 4, B>;
-    if (v == 4) return (void*)split_nee<true, 5, B>;
-    return (void*)split_nee<true, 6, B>;
+    if (v == 0) return (void*)split_nee<false, 4, M>;
+    if (v == 1) return (void*)split_nee<false, 5, M>;
+    if (v == 2) return (void*)split_nee<false, 6, M>;
+    if (v == 3) return (void*)split_nee<true, 4, M>;
+    if (v == 4) return (void*)split_nee<true, 5, M>;
+    return (void*)split_nee<true, 6, M>;
 }
 
 // One grid of resident blocks, no more than the slots fill.
@@ -597,30 +606,36 @@ static cudaError_t persistent(void* fn, const WaveArgs& a, int sms, cudaStream_t
     return cudaLaunchKernel(fn, dim3(std::min(blocks, (a.slots + threads - 1) / threads)), dim3(threads), args, 0, st);
 }
 
-// Batched launches (a.nframes > 0) have no counting build.
+// Batched launches (a.nframes > 0) have no counting build. NEE needs nothing
+// of a single frame's record.
+static Launch launch_of(const WaveArgs& a) { return !a.nframes ? PLAIN : (a.one_frame ? ONE_FRAME : FRAMES); }
+
 cudaError_t launch_split_logic(const WaveArgs& a, bool count, cudaStream_t st) {
     const unsigned blocks = (a.slots + LOGIC_THREADS - 1u) / LOGIC_THREADS;
-    if (a.nframes) {
-        if (count) return cudaErrorInvalidValue;
-        split_logic<false, true><<<blocks, LOGIC_THREADS, 0, st>>>(a);
-    } else if (count) {
-        split_logic<true, false><<<blocks, LOGIC_THREADS, 0, st>>>(a);
-    } else {
-        split_logic<false, false><<<blocks, LOGIC_THREADS, 0, st>>>(a);
-    }
+    const Launch m = launch_of(a);
+    if (m != PLAIN && count) return cudaErrorInvalidValue;
+    if (m == FRAMES) split_logic<false, FRAMES><<<blocks, LOGIC_THREADS, 0, st>>>(a);
+    else if (m == ONE_FRAME) split_logic<false, ONE_FRAME><<<blocks, LOGIC_THREADS, 0, st>>>(a);
+    else if (count) split_logic<true, PLAIN><<<blocks, LOGIC_THREADS, 0, st>>>(a);
+    else split_logic<false, PLAIN><<<blocks, LOGIC_THREADS, 0, st>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_split_shade(const WaveArgs& a, bool count, int variant, int sms, cudaStream_t st) {
     variant = variant < 0 ? 0 : (variant > 2 ? 2 : variant);
-    if (a.nframes) return count ? cudaErrorInvalidValue : persistent(shade_fn<false, true>(variant), a, sms, st, 128);
-    return persistent(count ? shade_fn<true, false>(variant) : shade_fn<false, false>(variant), a, sms, st, 128);
+    const Launch m = launch_of(a);
+    if (m != PLAIN && count) return cudaErrorInvalidValue;
+    void* fn = m == FRAMES ? shade_fn<false, FRAMES>(variant)
+               : m == ONE_FRAME ? shade_fn<false, ONE_FRAME>(variant)
+               : count ? shade_fn<true, PLAIN>(variant) : shade_fn<false, PLAIN>(variant);
+    return persistent(fn, a, sms, st, 128);
 }
 
 cudaError_t launch_split_nee(const WaveArgs& a, bool count, int variant, int sms, cudaStream_t st) {
     variant = variant < 0 ? 0 : (variant > 5 ? 5 : variant);
-    if (a.nframes) return count ? cudaErrorInvalidValue : persistent(nee_fn<true>(variant), a, sms, st, NEE_THREADS);
-    return persistent(nee_fn<false>(variant), a, sms, st, NEE_THREADS);
+    const Launch m = launch_of(a);
+    if (m != PLAIN && count) return cudaErrorInvalidValue;
+    return persistent(m == FRAMES ? nee_fn<FRAMES>(variant) : nee_fn<PLAIN>(variant), a, sms, st, NEE_THREADS);
 }
 
 #ifdef OXPT_FAST

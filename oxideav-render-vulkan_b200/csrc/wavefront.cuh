@@ -147,6 +147,8 @@ struct WaveArgs {
     // words): `s` is then that scene, for the traversal kernels' staged
     // top nodes
     uint32_t one_scene = 0u;
+    // a batch of one frame whose scene, but for the camera and the seed, is `s`
+    uint32_t one_frame = 0u;
     // continuation rays walk the four-wide tree (traversal variants 3-5;
     // the tolerance plan: closest hits equal except near-ties)
     uint32_t closest4 = 0u;

@@ -552,7 +552,7 @@ void* wide_fn(bool ext, int v) {
 // variant 0: 6 resident blocks per SM; 1 and 2: 8 (10 would leave 48
 // registers a thread, see above).
 cudaError_t launch_wide_walk(const WaveArgs& a, bool ext, int variant, int sd, int sms, cudaStream_t st) {
-    void* fn = a.nframes > 0 ? (sd <= 32 ? wide_fn<32, true>(ext, variant) : wide_fn<64, true>(ext, variant))
+    void* fn = a.nframes > 0 && !a.one_frame ? (sd <= 32 ? wide_fn<32, true>(ext, variant) : wide_fn<64, true>(ext, variant))
                              : (sd <= 32 ? wide_fn<32, false>(ext, variant) : wide_fn<64, false>(ext, variant));
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, NT, 0);
