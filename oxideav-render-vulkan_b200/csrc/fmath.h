@@ -143,12 +143,8 @@ FM_FN float fm_sin(float x) {
     int q;
     float r = fm_reduce_pio2(x, &q);
     float s = fm_sin_poly(r), c = fm_cos_poly(r);
-    switch (q) {
-        case 0: return s;
-        case 1: return c;
-        case 2: return -s;
-        default: return -c;
-    }
+    const float v = (q & 1) ? c : s;
+    return (q & 2) ? -v : v;
 }
 
 FM_FN float fm_cos(float x) {
@@ -159,12 +155,8 @@ FM_FN float fm_cos(float x) {
     int q;
     float r = fm_reduce_pio2(x, &q);
     float s = fm_sin_poly(r), c = fm_cos_poly(r);
-    switch (q) {
-        case 0: return c;
-        case 1: return -s;
-        case 2: return -c;
-        default: return s;
-    }
+    const float v = (q & 1) ? s : c;
+    return ((q + 1) & 2) ? -v : v;
 }
 
 // ---------------------------------------------------------------------

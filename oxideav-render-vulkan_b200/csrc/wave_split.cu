@@ -353,8 +353,88 @@ __global__ void __launch_bounds__(LOGIC_THREADS, 4) split_logic(const __grid_con
     }
 }
 
+// The radiance cache's part at a vertex; true when the path ends here, the
+// cache supplying the rest.
+__device__ __forceinline__ bool nrc_vertex(const WaveArgs& a, const Scene& s, uint32_t i, const PathCore& pc,
+                                           const Sampler& smp, const Vertex& vx, float t) {
+    bool spread_ok = true;
+    {
+        // Path spread (Mueller et al. 2021): a0 = t^2 / (4 pi |cos|) at the
+        // primary vertex, then the sum of sqrt(t^2 / (pdf |cos|)) over bounces.
+        const float cosv = fabsf(dot(vx.ng, pc.d));
+        float2 sp = pc.k == 0u ? make_float2(0.0f, 0.0f) : a.nrc.s_spread[i];
+        if (pc.k == 0u) sp.x = t * t / (4.0f * PI * fmaxf(cosv, 1e-6f));
+        else if (pc.prev_pdf > 0.0f && cosv > 0.0f) sp.y += sqrtf(t * t / (pc.prev_pdf * cosv));
+        a.nrc.s_spread[i] = sp;
+        spread_ok = a.nrc.spread <= 0.0f || sp.y * sp.y > a.nrc.spread * sp.x;
+    }
+    const uint32_t tail = a.nrc.s_tail[i];
+    if (tail == pc.k && (smp.path_seed & a.nrc.train_mask) == 0u) {
+        // A training path's suffix ends here, into the cache.
+        float4 f[3];
+        nrc_features(s, vx, f);
+        uint32_t q = atomicAdd(&a.nrc.counts[0], 1u);
+        if (q < a.nrc.q_cap) {
+            a.nrc.q_in[3 * (size_t)q] = f[0];
+            a.nrc.q_in[3 * (size_t)q + 1] = f[1];
+            a.nrc.q_in[3 * (size_t)q + 2] = f[2];
+            a.nrc.q_beta[q] = make_float4(pc.beta.x, pc.beta.y, pc.beta.z, 0.0f);
+            a.nrc.q_item[q] = a.st.item[i];
+            uint32_t ti = a.nrc.s_tidx[i];
+            if (ti != NONE) {
+                float4 b0 = a.nrc.s_beta[i];
+                float rx = b0.x > 0.0f ? pc.beta.x / b0.x : 0.0f;
+                float ry = b0.y > 0.0f ? pc.beta.y / b0.y : 0.0f;
+                float rz = b0.z > 0.0f ? pc.beta.z / b0.z : 0.0f;
+                a.nrc.t_tail[ti] = make_uint4(q, __float_as_uint(rx), __float_as_uint(ry), __float_as_uint(rz));
+            }
+        }
+        a.st.nee_n[i] = 0u;
+        return true;
+    }
+    if (pc.k >= a.nrc.query_k && tail == NONE && spread_ok) {
+        float4 f[3];
+        nrc_features(s, vx, f);
+        if ((smp.path_seed & a.nrc.train_mask) != 0u) {
+            // A rendering path ends here: the cache supplies the rest.
+            uint32_t q = atomicAdd(&a.nrc.counts[0], 1u);
+            if (q < a.nrc.q_cap) {
+                a.nrc.q_in[3 * (size_t)q] = f[0];
+                a.nrc.q_in[3 * (size_t)q + 1] = f[1];
+                a.nrc.q_in[3 * (size_t)q + 2] = f[2];
+                a.nrc.q_beta[q] = make_float4(pc.beta.x, pc.beta.y, pc.beta.z, 0.0f);
+                a.nrc.q_item[q] = a.st.item[i];
+            }
+            a.st.nee_n[i] = 0u;
+            return true;
+        }
+        a.nrc.s_tail[i] = a.nrc.suffix ? pc.k + a.nrc.suffix : 0xfffffffeu;
+        uint32_t ti = atomicAdd(&a.nrc.counts[1], 1u);
+        if (ti < a.nrc.t_cap) {
+            a.nrc.t_in[3 * (size_t)ti] = f[0];
+            a.nrc.t_in[3 * (size_t)ti + 1] = f[1];
+            a.nrc.t_in[3 * (size_t)ti + 2] = f[2];
+            a.nrc.t_target[ti] = make_float4(0.f, 0.f, 0.f, 0.f);
+            a.nrc.t_tail[ti] = make_uint4(NONE, 0u, 0u, 0u);
+            a.nrc.s_pre[i] = make_float4(pc.radiance.x, pc.radiance.y, pc.radiance.z, 0.0f);
+            a.nrc.s_beta[i] = make_float4(pc.beta.x, pc.beta.y, pc.beta.z, 0.0f);
+            a.nrc.s_tidx[i] = ti;
+        }
+    }
+    return false;
+}
+
+// Bound by fetching instructions: of 22 cycles an instruction, 12 waited for
+// the next one (ncu, 1080p materials scene with a radiance cache). So a block
+// is 256 threads and stays together: its warps meet before a hit is shaded,
+// before the vertex is stored and before the path is continued, and fetch each
+// part once (against 128 threads that met once a round, for 8 spp of the
+// 1.05 M-triangle frame / of 480 k-triangle boxes: 3.59 to 3.37 / 3.70 to
+// 3.34 ms; 512 threads: 3.53 / 3.42).
+constexpr uint32_t SHADE_THREADS = 256u;
+
 template <bool COUNT, int MINB, int M>
-__global__ void __launch_bounds__(128, MINB) split_shade(const __grid_constant__ WaveArgs a) {
+__global__ void __launch_bounds__(SHADE_THREADS, MINB) split_shade(const __grid_constant__ WaveArgs a) {
     __shared__ uint32_t s_dirs[128];
     __shared__ uint4 s_sobol[128];
     __shared__ float s_sheen[512];
@@ -368,98 +448,41 @@ __global__ void __launch_bounds__(128, MINB) split_shade(const __grid_constant__
     const uint32_t n = *((volatile uint32_t*)&a.ctr[3]);
     unsigned long long shaded = 0;
     for (uint32_t q0 = blockIdx.x * blockDim.x; q0 < n; q0 += gridDim.x * blockDim.x) {
-        __syncthreads();  // the block's warps fetch the same code together
-        uint32_t q = q0 + threadIdx.x;
-        if (q >= n) continue;
-        uint32_t i = a.q.shade[q];
-        const Scene& s = slot_scene<M>(a, i);
+        __syncthreads();
+        const uint32_t q = q0 + threadIdx.x;
+        uint32_t i = 0u;
         PathCore pc;
         Sampler smp;
-        load_state(a, i, &pc, &smp);
-        uint32_t hmat;
-        Hit hit = load_hit(a, i, &hmat);
         Vertex vx;
-        int r = shade_hit<COUNT>(s, M == ONE_FRAME ? a.frames[0].s : s, s_sheen, s_sobol, smp, pc, hit, hmat, &vx, &shaded);
-        if (r != PATH_VERTEX) {
-            save_rad(a, i, pc, ST_ENDING);
-            continue;
+        bool vertex = false;
+        if (q < n) {
+            i = a.q.shade[q];
+            const Scene& s = slot_scene<M>(a, i);
+            load_state(a, i, &pc, &smp);
+            uint32_t hmat;
+            Hit hit = load_hit(a, i, &hmat);
+            const int r = shade_hit<COUNT>(s, M == ONE_FRAME ? a.frames[0].s : s, s_sheen, s_sobol, smp, pc, hit, hmat,
+                                           &vx, &shaded);
+            vertex = r == PATH_VERTEX && (!a.nrc.on || !nrc_vertex(a, s, i, pc, smp, vx, hit.t));
+            if (!vertex) save_rad(a, i, pc, ST_ENDING);
         }
-        bool spread_ok = true;
-        if (a.nrc.on) {
-            // Path spread (Mueller et al. 2021): a0 = t^2 / (4 pi |cos|) at the
-            // primary vertex, then the sum of sqrt(t^2 / (pdf |cos|)) over bounces.
-            const float cosv = fabsf(dot(vx.ng, pc.d));
-            float2 sp = pc.k == 0u ? make_float2(0.0f, 0.0f) : a.nrc.s_spread[i];
-            if (pc.k == 0u) sp.x = hit.t * hit.t / (4.0f * PI * fmaxf(cosv, 1e-6f));
-            else if (pc.prev_pdf > 0.0f && cosv > 0.0f) sp.y += sqrtf(hit.t * hit.t / (pc.prev_pdf * cosv));
-            a.nrc.s_spread[i] = sp;
-            spread_ok = a.nrc.spread <= 0.0f || sp.y * sp.y > a.nrc.spread * sp.x;
+        __syncthreads();
+        if (vertex) {
+            const Scene& s = slot_scene<M>(a, i);
+            uint32_t v = append1(&a.ctr[4]);
+            put_vertex(a, v, vx, pc, smp.path_seed);
+            a.q.vslot[v] = i;
+            const uint32_t jobs = M == FRAMES ? s.P.cfg[2] + 1u : a.jobs;
+            a.st.nee_n[i] = jobs;
+            if (a.st.vis) a.st.vis[i] = 0u;
+            const uint32_t kind = sampled_light(s, vx.pl_u.z);
+            if (kind == SAMPLED_ENV) a.q.vlight[append1(&a.ctr[11])] = v;
+            else if (kind == SAMPLED_AREA) a.q.vlight[a.vcap - 1u - append1(&a.ctr[12])] = v;
+            else if (!a.st.vis) a.st.pend[(uint64_t)i * a.jobs + jobs - 1u] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        const uint32_t tail = a.nrc.on ? a.nrc.s_tail[i] : NONE;
-        if (a.nrc.on && tail == pc.k && (smp.path_seed & a.nrc.train_mask) == 0u) {
-            // A training path's suffix ends here, into the cache.
-            float4 f[3];
-            nrc_features(s, vx, f);
-            uint32_t q = atomicAdd(&a.nrc.counts[0], 1u);
-            if (q < a.nrc.q_cap) {
-                a.nrc.q_in[3 * (size_t)q] = f[0];
-                a.nrc.q_in[3 * (size_t)q + 1] = f[1];
-                a.nrc.q_in[3 * (size_t)q + 2] = f[2];
-                a.nrc.q_beta[q] = make_float4(pc.beta.x, pc.beta.y, pc.beta.z, 0.0f);
-                a.nrc.q_item[q] = a.st.item[i];
-                uint32_t ti = a.nrc.s_tidx[i];
-                if (ti != NONE) {
-                    float4 b0 = a.nrc.s_beta[i];
-                    float rx = b0.x > 0.0f ? pc.beta.x / b0.x : 0.0f;
-                    float ry = b0.y > 0.0f ? pc.beta.y / b0.y : 0.0f;
-                    float rz = b0.z > 0.0f ? pc.beta.z / b0.z : 0.0f;
-                    a.nrc.t_tail[ti] = make_uint4(q, __float_as_uint(rx), __float_as_uint(ry), __float_as_uint(rz));
-                }
-            }
-            a.st.nee_n[i] = 0u;
-            save_rad(a, i, pc, ST_ENDING);
-            continue;
-        }
-        if (a.nrc.on && pc.k >= a.nrc.query_k && tail == NONE && spread_ok) {
-            float4 f[3];
-            nrc_features(s, vx, f);
-            if ((smp.path_seed & a.nrc.train_mask) != 0u) {
-                // A rendering path ends here: the cache supplies the rest.
-                uint32_t q = atomicAdd(&a.nrc.counts[0], 1u);
-                if (q < a.nrc.q_cap) {
-                    a.nrc.q_in[3 * (size_t)q] = f[0];
-                    a.nrc.q_in[3 * (size_t)q + 1] = f[1];
-                    a.nrc.q_in[3 * (size_t)q + 2] = f[2];
-                    a.nrc.q_beta[q] = make_float4(pc.beta.x, pc.beta.y, pc.beta.z, 0.0f);
-                    a.nrc.q_item[q] = a.st.item[i];
-                }
-                a.st.nee_n[i] = 0u;
-                save_rad(a, i, pc, ST_ENDING);
-                continue;
-            }
-            a.nrc.s_tail[i] = a.nrc.suffix ? pc.k + a.nrc.suffix : 0xfffffffeu;
-            uint32_t ti = atomicAdd(&a.nrc.counts[1], 1u);
-            if (ti < a.nrc.t_cap) {
-                a.nrc.t_in[3 * (size_t)ti] = f[0];
-                a.nrc.t_in[3 * (size_t)ti + 1] = f[1];
-                a.nrc.t_in[3 * (size_t)ti + 2] = f[2];
-                a.nrc.t_target[ti] = make_float4(0.f, 0.f, 0.f, 0.f);
-                a.nrc.t_tail[ti] = make_uint4(NONE, 0u, 0u, 0u);
-                a.nrc.s_pre[i] = make_float4(pc.radiance.x, pc.radiance.y, pc.radiance.z, 0.0f);
-                a.nrc.s_beta[i] = make_float4(pc.beta.x, pc.beta.y, pc.beta.z, 0.0f);
-                a.nrc.s_tidx[i] = ti;
-            }
-        }
-        uint32_t v = append1(&a.ctr[4]);
-        put_vertex(a, v, vx, pc, smp.path_seed);
-        a.q.vslot[v] = i;
-        const uint32_t jobs = M == FRAMES ? s.P.cfg[2] + 1u : a.jobs;
-        a.st.nee_n[i] = jobs;
-        if (a.st.vis) a.st.vis[i] = 0u;
-        const uint32_t kind = sampled_light(s, vx.pl_u.z);
-        if (kind == SAMPLED_ENV) a.q.vlight[append1(&a.ctr[11])] = v;
-        else if (kind == SAMPLED_AREA) a.q.vlight[a.vcap - 1u - append1(&a.ctr[12])] = v;
-        else if (!a.st.vis) a.st.pend[(uint64_t)i * a.jobs + jobs - 1u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncthreads();
+        if (!vertex) continue;
+        const Scene& s = slot_scene<M>(a, i);
         f3 o;
         if (continue_path(s, s_sheen, s_sobol, smp, pc, vx, &o)) {
             a.st.seed[i].w = pc.k;
@@ -577,14 +600,13 @@ __global__ void __launch_bounds__(NEE_THREADS, MINB * 128 / NEE_THREADS) split_n
     }
 }
 
-// Variants: shade kernel for 5 (0, 1) or 6 blocks of 128 threads per SM (96
-// registers: 3.95 ms of shading per 8 spp of the 1.05 M-triangle frame against
-// 4.3 at 4 blocks; left more registers the compiler took up to 178 and the
-// kernel 5 to 6.9 ms); the NEE kernel job-major (0-2) or vertex-major (3-5)
-// for 4 / 5 / 6 blocks of 128.
+// Variants: shade kernel for 2 (0, 1; 128 registers) or 3 (2; 80) blocks per
+// SM, 3.37 against 3.26 ms of shading per 8 spp of the 1.05 M-triangle frame,
+// 3.34 against 3.71 of 480 k-triangle boxes; the NEE kernel job-major (0-2) or
+// vertex-major (3-5) for 4 / 5 / 6 blocks of 128.
 template <bool C, int M>
 static void* shade_fn(int v) {
-    return v < 2 ? (void*)split_shade<C, 5, M> : (void*)split_shade<C, 6, M>;
+    return v < 2 ? (void*)split_shade<C, 2, M> : (void*)split_shade<C, 3, M>;
 }
 template <int M>
 static void* nee_fn(int v) {
@@ -628,7 +650,7 @@ cudaError_t launch_split_shade(const WaveArgs& a, bool count, int variant, int s
     void* fn = m == FRAMES ? shade_fn<false, FRAMES>(variant)
                : m == ONE_FRAME ? shade_fn<false, ONE_FRAME>(variant)
                : count ? shade_fn<true, PLAIN>(variant) : shade_fn<false, PLAIN>(variant);
-    return persistent(fn, a, sms, st, 128);
+    return persistent(fn, a, sms, st, SHADE_THREADS);
 }
 
 cudaError_t launch_split_nee(const WaveArgs& a, bool count, int variant, int sms, cudaStream_t st) {
