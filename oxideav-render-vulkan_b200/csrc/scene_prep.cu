@@ -228,18 +228,7 @@ class Stager {
   public:
     explicit Stager(cudaStream_t st) : st_(st) {}
     ~Stager() { release(); }
-    cudaError_t init() {
-        for (int i = 0; i < 2; i++) {
-            cudaError_t e = PinnedPool::get().take(&buf_[i], CHUNK);
-            if (e != cudaSuccess) {
-                buf_[i] = nullptr;
-                return e;
-            }
-            e = cudaEventCreateWithFlags(&ev_[i], cudaEventDisableTiming);
-            if (e != cudaSuccess) return e;
-        }
-        return cudaSuccess;
-    }
+    cudaError_t init() { return take(); }
     cudaError_t put(const void* region, void* dst, const void* src, size_t bytes) {
         char* d = (char*)dst;
         const char* s = (const char*)src;
@@ -278,6 +267,17 @@ class Stager {
 
   private:
     static constexpr size_t CHUNK = 32u << 20;
+    // The second chunk is taken when the first is full: pinning one is 15 ms
+    // of a process's first upload, and most scenes' textures and meshes,
+    // which are staged at the same time, fit one chunk each.
+    cudaError_t take() {
+        cudaError_t e = PinnedPool::get().take(&buf_[cur_], CHUNK);
+        if (e != cudaSuccess) {
+            buf_[cur_] = nullptr;
+            return e;
+        }
+        return cudaEventCreateWithFlags(&ev_[cur_], cudaEventDisableTiming);
+    }
     cudaError_t issue() {
         if (!run_len_) return cudaSuccess;
         cudaError_t e = cudaMemcpyAsync(run_dst_, buf_[cur_] + run_off_, run_len_, cudaMemcpyHostToDevice, st_);
@@ -290,6 +290,7 @@ class Stager {
         if ((e = cudaEventRecord(ev_[cur_], st_)) != cudaSuccess) return e;
         used_[cur_] = true;
         cur_ ^= 1;
+        if (!buf_[cur_] && (e = take()) != cudaSuccess) return e;
         if (used_[cur_] && (e = cudaEventSynchronize(ev_[cur_])) != cudaSuccess) return e;
         fill_ = 0;
         return cudaSuccess;
