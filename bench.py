@@ -1084,14 +1084,15 @@ def main():
     bytes_per_path = (BYTES_AABB * c[3] + BYTES_TRI * c[5] + (BYTES_ATTR + BYTES_MAT) * c[6]) / npaths
     kernel_bytes = {  # algorithmic bytes per camera path, per kernel
         "trace_paths": bytes_per_path,
-        "wave_logic": (BYTES_ATTR + BYTES_MAT) * c[6] / npaths,
         "wave_extend": (BYTES_AABB * h0[3] + BYTES_TRI * h0[5]) / npaths,
         "wave_shadow": (BYTES_AABB * h1[3] + BYTES_TRI * h1[5]) / npaths,
         "split_logic": 0.0,
         "split_shade": (BYTES_ATTR + BYTES_MAT) * c[6] / npaths,
         "split_nee": 0.0,
     }
-    kernel_bytes["walk_extend"] = kernel_bytes["wave_extend"]  # on-chip-stack kernels (trace_variant 3-5)
+    # trace_variant 3-5: the reference walk's bytes, whatever the wide walk reads
+    # for the same answers (64 bytes for four children)
+    kernel_bytes["walk_extend"] = kernel_bytes["wave_extend"]
     kernel_bytes["walk_shadow"] = kernel_bytes["wave_shadow"]
     rays_per_path = (c[1] + c[2]) / npaths
 
@@ -1167,9 +1168,8 @@ def main():
     mode = pt.tuning().mode
     walk = pt.tuning().trace_variant >= 3
     ext_name, sh_name = ("walk_extend", "walk_shadow") if walk else ("wave_extend", "wave_shadow")
-    kinds = {0: ((0, "trace_paths"),), 1: ((2, "wave_logic"), (3, ext_name), (4, sh_name)),
-             2: ((2, "split_logic"), (5, "split_shade"), (6, "split_nee"), (3, ext_name),
-                 (4, sh_name))}[mode]
+    wave_kinds = ((2, "split_logic"), (5, "split_shade"), (6, "split_nee"), (3, ext_name), (4, sh_name))
+    kinds = {0: ((0, "trace_paths"),), 1: wave_kinds, 2: wave_kinds}[mode]
     traffic_db = {}
     tf = ROOT / "profiles" / "traffic.json"
     if tf.exists():
@@ -1294,7 +1294,7 @@ def main():
                              "l1_l2_served_share": (1.0 - kd["traffic_bytes_per_launch"] /
                                                     kd["algorithmic_bytes_per_launch"]
                                                     if kd["traffic_bytes_per_launch"] else None),
-                             "limiter": "dependent-load latency and SIMD divergence of the walks: node and "
+                             "limiter": "instruction issue of the walks (about 77% of cycles): node and "
                                         "triangle bytes are served mostly by L1/L2 (see l1_l2_served_share), "
                                         "so frac is an effective bandwidth against the HBM copy peak, and "
                                         "dram_frac the kernel's real HBM use",

@@ -139,8 +139,9 @@ oxpt_status oxpt_diag_set_l2_window(oxpt_ctx* ctx, int on, uint64_t* granted);
  *                  round; the result buffer holds 16 bytes per path of a
  *                  round); check_every its bounces between completion
  *                  checks.
- *   shade_variant  surface shading kernel compiled for 5 (0, 1) or 6 (2)
- *                  resident blocks per SM: registers against occupancy.
+ *   shade_variant  surface shading kernel compiled for 2 (0, 1) or 3 (2)
+ *                  resident blocks of 256 threads per SM: registers against
+ *                  occupancy.
  *   trace_variant  wavefront traversal kernels: 0-2 with local-memory walk
  *                  stacks for 6 / 8 / 10 blocks per SM; 3-5 on the wide tree
  *                  (same results) for 6 / 8 / 8 blocks, or, for counting

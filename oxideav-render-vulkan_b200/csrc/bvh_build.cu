@@ -3,14 +3,16 @@
 // 32 bins per axis, unit SAH costs, leaves of at most 8 triangles).
 //
 // Per level of the tree:
-//   decide_small   one thread per node of at most LARGE triangles: bounds,
-//                  binning and the SAH sweep exactly as the host writes
-//                  them, then the stable partition of its triangle ids;
+//   decide_small   eight lanes per node of at most SMALL_MAX triangles:
+//                  bounds, binning and the SAH sweep with the host's bits,
+//                  then the stable partition of its triangle ids;
+//   decide_warp    a warp per node of at most LARGE triangles;
 //   decide_large   one CTA per larger node: bounds and bins reduced in
 //                  shared memory (float min / max as order-preserving
 //                  integers, so any order gives the host's bits), the SAH
 //                  sweep by one thread, then a stable partition chunk by
-//                  chunk with block scans;
+//                  chunk with block scans (above HUGE_N triangles: one CTA
+//                  per CHUNK of them);
 //   scan / emit    child pairs are numbered by an exclusive scan over the
 //                  level's split flags in node order (the host allocates
 //                  them in that order), node words are written and the next
