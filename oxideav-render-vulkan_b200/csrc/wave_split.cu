@@ -424,8 +424,9 @@ __device__ __forceinline__ bool nrc_vertex(const WaveArgs& a, const Scene& s, ui
     return false;
 }
 
-// Bound by fetching instructions: of 22 cycles an instruction, 12 waited for
-// the next one (ncu, 1080p materials scene with a radiance cache). So a block
+// Was bound by fetching instructions: of 22 cycles an instruction, 12 waited
+// for the next one (ncu, 1080p materials scene with a radiance cache; now half
+// a cycle, and load latency, 5.4 of 11.7 cycles, is the bound). So a block
 // is 256 threads and stays together: its warps meet before a hit is shaded,
 // before the vertex is stored and before the path is continued, and fetch each
 // part once (against 128 threads that met once a round, for 8 spp of the
