@@ -57,12 +57,20 @@ namespace {
 constexpr uint32_t NT = WAVE_TRAVERSE_THREADS;
 constexpr unsigned FULL = 0xffffffffu;
 constexpr uint32_t LEAF_BIT = 0x80000000u;
+constexpr uint32_t NOT_WALKED = 0xfffffffeu;  // for a hit: leave the ray to the reference's walk
 constexpr uint32_t LEAFCAP = 8;   // leaves a lane may have pending
 constexpr uint32_t SS = 6;        // stack entries a lane keeps in shared memory
 constexpr uint32_t FLUSH = 32;    // pending leaves of a warp that start a pass of triangle tests
 constexpr uint32_t MIN_RAYS = 4;  // rays of a warp, at least, when they are few
 constexpr int STEPS = 4;          // node steps between checks
 constexpr float ETA = 3.8146973e-6f;     // 2^-18
+// Reciprocal directions are cut to INV_MAX, so that the product with a node's
+// corner (up to 260 times the largest coordinate below the box) stays finite
+// for coordinates up to FAR. The rays this changes move less than 10^-17 of a
+// distance along the axis, and eta x INV_MAX is still 10^11 times the largest
+// coordinate, so the box test stays on the safe side.
+constexpr float INV_MAX = 1.0e17f;
+constexpr float FAR = 1.0e18f;
 constexpr float LIMIT = 1.00002f;        // closest hit: distance limit over the best distance
 
 // One warp's rays and pending work in shared memory.
@@ -120,21 +128,22 @@ struct NodeRay {
     float inv[3], nb[3], c[3];
 };
 
-__device__ __forceinline__ NodeRay node_ray(const Scene& s, const Ray& r) {
+// False when the coordinates are out of the node step's range.
+__device__ __forceinline__ bool node_ray(const Scene& s, const Ray& r, NodeRay& n) {
     float4 lo = geomv(s, 0), hi = geomv(s, 1);
     float m = fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(hi.x)), fmaxf(fabsf(lo.y), fabsf(hi.y))),
                     fmaxf(fabsf(lo.z), fabsf(hi.z)));
     m = fmaxf(m, fmaxf(fabsf(r.o.x), fmaxf(fabsf(r.o.y), fabsf(r.o.z))));
     const float eta = m * ETA;
-    NodeRay n;
     const float iv[3] = {r.inv.x, r.inv.y, r.inv.z}, oo[3] = {r.o.x, r.o.y, r.o.z};
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        n.inv[a] = iv[a];
-        n.nb[a] = -((iv[a] < 0.0f ? oo[a] - eta : oo[a] + eta) * iv[a]);
-        n.c[a] = fabsf(2.0f * eta * iv[a]);
+        const float v = fminf(fmaxf(iv[a], -INV_MAX), INV_MAX);
+        n.inv[a] = v;
+        n.nb[a] = -((v < 0.0f ? oo[a] - eta : oo[a] + eta) * v);
+        n.c[a] = fabsf(2.0f * eta * v);
     }
-    return n;
+    return m <= FAR;
 }
 
 // Byte k of w as the float 32768 + byte.
@@ -293,20 +302,27 @@ __device__ __forceinline__ void finish(const WaveArgs& a, WarpMem<EXT>& M, uint3
     const Scene& s = ray_scene<EXT, BATCH>(a, src);
     const float4 o = M.o[lane], d = EXT ? a.st.dir[src] : a.q.sh_d[src];
     const Ray r = make_ray(xyz(o), xyz(d));
-    const uint32_t ln = __ldg(s.leaf_of + tri);
-    const float e = slab(r, geomv(s, 2ull * ln), geomv(s, 2ull * ln + 1u), EXT ? INF : o.w);
+    float e = -1.0f;
+    if (tri != NOT_WALKED) {
+        const uint32_t ln = __ldg(s.leaf_of + tri);
+        e = slab(r, geomv(s, 2ull * ln), geomv(s, 2ull * ln + 1u), EXT ? INF : o.w);
+    }
     Hit h;
     uint32_t mat;
     if (EXT) {
-        const uint64_t tb = tri_base(s, tri);
-        const float4 q0 = geomv(s, tb), q1 = geomv(s, tb + 1), q2 = geomv(s, tb + 2);
-        bool got = intersect(r, q0, q1, q2, INF, &h);
-        h.slot = tri;
-        mat = __float_as_uint(q2.w);
-        // The second distance as a float: a NaN when there is none, so that
-        // "not at or below" holds.
-        const float t = h.t, sec = __uint_as_float(M.second[lane]);
-        const bool sure = got && e >= 0.0f && (e <= t ? !(sec <= t) : (!(sec <= e) && e < tl));
+        bool sure = e >= 0.0f;
+        if (sure) {
+            const uint64_t tb = tri_base(s, tri);
+            const float4 q0 = geomv(s, tb), q1 = geomv(s, tb + 1), q2 = geomv(s, tb + 2);
+            sure = intersect(r, q0, q1, q2, INF, &h);
+            h.slot = tri;
+            mat = __float_as_uint(q2.w);
+            // The second distance as a float: a NaN when there is none, so that
+            // "not at or below" holds.
+            const float t = h.t, sec = __uint_as_float(M.second[lane]);
+            sure = sure && (e <= t ? !(sec <= t) : (!(sec <= e) && e < tl));
+        }
+        bool got = sure;
         if (!sure) {
             const uint4 sd = a.st.seed[src];
             got = reference_walk(&s, &r, INF, sd.z, sd.w << 16u, sd.w == 0u, false, NONE, &h, &mat, a.err);
@@ -380,7 +396,7 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
                     const Scene& s = ray_scene<EXT, BATCH>(a, src);
                     const Ray r = make_ray(xyz(o), xyz(d));
                     if (r.valid && s.bvh4_root != NONE && s.P.env[3] != 0u) {
-                        nr = node_ray(s, r);
+                        const bool walk = node_ray(s, r, nr);
                         if (BATCH) nodes = reinterpret_cast<const char*>(s.wide);
                         M.o[lane] = o;
                         M.shear[lane] = make_float4(r.shear.x, r.shear.y, r.shear.z,
@@ -388,17 +404,17 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
                                                                     (primary ? 64u : 0u)));
                         M.src[lane] = src;
                         if (EXT) {
-                            M.best[lane] = ~0ull;
+                            M.best[lane] = walk ? ~0ull : NOT_WALKED;
                             M.second[lane] = 0xffffffffu;
                         } else {
-                            M.found[lane] = NONE;
+                            M.found[lane] = walk ? NONE : NOT_WALKED;
                         }
                         tl = o.w;
                         sp = group = 0u;
                         if (!EXT) group = s.bvh4_root << 4 | 1u;
                         guard = 4u * STEPS * min(s.bvh4_nodes, 1u << 27) + 64u;
-                        cur = s.bvh4_root;
-                        if (cur & LEAF_BIT) {  // a tree of one leaf
+                        cur = walk ? s.bvh4_root : NONE;
+                        if (walk && (cur & LEAF_BIT)) {  // a tree of one leaf
                             M.leaf[0][lane] = cur;
                             leaves = 1u;
                             cur = NONE;
