@@ -54,9 +54,10 @@ static __device__ f3 perturb(const Scene& s, uint32_t slot, f3 b, f3 n, float4 t
 }
 
 // Four words of a material record from word `k` (a multiple of 4): one load
-// where the records are 16-byte aligned (as the host layer lays them out).
+// where the record's address is a multiple of 16 (as in the buffers of a
+// context; a caller's own buffer may start at any word), else a word at a time.
 __device__ __forceinline__ float4 mat4(const Scene& s, uint32_t o, uint32_t k) {
-    if ((o & 3u) == 0u) {
+    if (((uint32_t)(uintptr_t)(s.tables + o) & 15u) == 0u) {
         const uint32_t i = o + k;
         return (uint64_t)i + 4u <= s.table_words ? __ldg(reinterpret_cast<const float4*>(s.tables + i))
                                                  : tv4(s, i);
