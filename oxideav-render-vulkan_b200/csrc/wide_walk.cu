@@ -28,13 +28,20 @@
 // Why the result is the reference walk's although the order and the box
 // test are not:
 // * Boxes are widened by eta = 2^-18 x the largest coordinate of the scene
-//   box and the ray origin. With u = 2^-24 the watertight test places the
-//   hit point within 46 u of that coordinate from the ray, and what the
-//   slab arithmetic below loses is within 8 u of it and within 1/128
-//   of a byte step (the bytes leave 1/32), so a triangle that passes the
-//   triangle test at distance t has t between the widened entry and exit
-//   distances of every box around it: with a distance limit T, all triangles
-//   with t <= T are tested, in whatever order the boxes come.
+//   box and the ray origin. With u = 2^-24, what the slab arithmetic below
+//   loses is within 8 u of that and within 1/128 of a byte step (the bytes
+//   leave 1/32): every box that the exact test enters is entered here too.
+// * A closest hit's distance limit T is compared with the entry on the ray's
+//   dominant axis alone. The watertight test's distance is a weighted mean of
+//   its vertices' distances on that axis, whatever the weights are, so it is
+//   at least the box's entry there (but for some u of itself, less than the
+//   2e-5 that T leaves): all triangles with t <= T are tested, in whatever
+//   order the boxes come. On the other axes no such bound holds: where a
+//   triangle's projection is thin against the rounding of its vertices, the
+//   weights are noise and the hit lies anywhere in the triangle, also before
+//   the ray enters its box. (Culling by the entry on all three axes took 10%
+//   less time and could lose such a hit to one behind it. Projections of an
+//   area below 1e-30, where products of the test underflow, are not covered.)
 // * Any hit: the reference accepts a triangle when its leaf's exact box test
 //   passes (a box passes whenever a box inside it does: checked on upload),
 //   so an accepted triangle is checked against its leaf's exact box once.
@@ -358,10 +365,11 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
     bool active = false;                 // the lane holds a ray
     uint32_t cur = NONE;                 // next node (NONE: none left)
     uint32_t group = 0u, sp = 0u;        // siblings still to visit, and the groups above them on the stack
-    float group_t = 0.0f;                // closest: smallest entry distance of the group
+    float group_t = 0.0f;                // closest: smallest entry of the group on the dominant axis
     uint32_t leaves = 0u;                // leaves pending
     uint32_t guard = 0u;
     float tl = 0.0f;                     // distance limit
+    uint32_t kz = 0u;                    // closest: the ray's dominant axis
     const char* nodes = reinterpret_cast<const char*>(a.s.wide);
     NodeRay nr;
     uint32_t deep[SD];                   // stack entries from SS on
@@ -410,6 +418,7 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
                             M.found[lane] = walk ? NONE : NOT_WALKED;
                         }
                         tl = o.w;
+                        kz = r.kz;
                         sp = group = 0u;
                         if (!EXT) group = s.bvh4_root << 4 | 1u;
                         guard = 4u * STEPS * min(s.bvh4_nodes, 1u << 27) + 64u;
@@ -450,6 +459,7 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
             const char* nd = nodes + (uint64_t)cur * 64u;
             const u8x v0 = ld32(nd), v1 = ld32(nd + 32);
             float t0[4], t1[4], tx[4], ty[4];
+            float td[4];  // closest: entry on the ray's dominant axis
 #pragma unroll
             for (int ax = 0; ax < 3; ax++) {
                 const float A = __uint_as_float(v0.v[3 + ax]) * nr.inv[ax];
@@ -464,13 +474,17 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
                                           make_float2(bn, bf));
                     if (ax == 0) t0[k] = t.x, t1[k] = t.y;
                     else if (ax == 1) tx[k] = t.x, ty[k] = t.y;
-                    else t0[k] = max3(fmaxf(t0[k], 0.0f), tx[k], t.x), t1[k] = min3(fminf(t1[k], tl), ty[k], t.y);
+                    else {
+                        if (EXT) td[k] = kz == 0u ? t0[k] : (kz == 1u ? tx[k] : t.x);
+                        t0[k] = max3(fmaxf(t0[k], 0.0f), tx[k], t.x);
+                        t1[k] = min3(EXT ? t1[k] : fminf(t1[k], tl), ty[k], t.y);
+                    }
                 }
             }
             uint32_t hit = 0u;
 #pragma unroll
             for (int k = 0; k < 4; k++)
-                if (t0[k] <= t1[k]) hit |= 1u << k;
+                if (t0[k] <= t1[k] && (!EXT || td[k] <= tl)) hit |= 1u << k;
             const uint32_t inner = hit & v0.v[3], leaf = hit & v0.v[4];  // the low four bits
 #pragma unroll
             for (int k = 0; k < 4; k++)
@@ -494,23 +508,23 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
                 for (int k = 0; k < 4; k++)
                     key[k] = (inner & (1u << k)) ? ((__float_as_uint(t0[k]) & ~3u) | (uint32_t)k) : NONE;
                 const uint32_t lo01 = min(key[0], key[1]), lo23 = min(key[2], key[3]);
-                const uint32_t nk = EXT ? min(lo01, lo23) & 3u : (uint32_t)__ffs(inner) - 1u;
+                const uint32_t nk = min(lo01, lo23) & 3u;
                 const uint32_t rest = inner & ~(1u << nk), base = v1.v[4];
                 if (rest) {
                     if (group & 15u) {
                         if (sp < SS) {
                             M.stack[sp][lane] = group;
-                            if (EXT) M.stack_t[sp][lane] = group_t;
+                            M.stack_t[sp][lane] = group_t;
                         } else {
                             deep[sp] = group;
-                            if (EXT) deep_t[sp] = group_t;
+                            deep_t[sp] = group_t;
                         }
                         sp++;
                     }
                     group = base << 4 | rest;
-                    if (EXT)  // the second smallest key
-                        group_t = __uint_as_float(
-                            min(max(lo01, lo23), lo01 < lo23 ? max(key[0], key[1]) : max(key[2], key[3])) & ~3u);
+                    group_t = INF;
+#pragma unroll
+                    for (int k = 0; k < 4; k++) group_t = fminf(group_t, rest & (1u << k) ? td[k] : INF);
                 }
                 cur = base + nk;
             } else {
@@ -520,9 +534,9 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
                         if (sp == 0u) break;
                         sp--;
                         group = sp < SS ? M.stack[sp][lane] : deep[sp];
-                        if (EXT) group_t = sp < SS ? M.stack_t[sp][lane] : deep_t[sp];
+                        group_t = sp < SS ? M.stack_t[sp][lane] : deep_t[sp];
                     }
-                    if (EXT && group_t > tl) {
+                    if (group_t > tl) {
                         group = 0u;
                         continue;
                     }
