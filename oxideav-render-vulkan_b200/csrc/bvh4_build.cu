@@ -284,9 +284,15 @@ __global__ void depth_level(const uint32_t* frontier, uint32_t K, const uint32_t
 // the y step which are leaves. The corner is that of byte value -32768, since
 // the walk reads a byte q as the float 32768 + q. Boxes are rounded outwards
 // by at least 1/32 of a step (more than the walk's arithmetic loses on them).
-__global__ void wide_nodes(const uint4* bvh4, uint32_t n4, uint32_t* out) {
+// A step is at least 2.5e-7 of the node's largest coordinate, so that rounding
+// the corner moves the planes by less than half a step, and 2^-40 of the
+// scene's (the walk's bound on cut reciprocals).
+__global__ void wide_nodes(const uint32_t* words, const uint4* bvh4, uint32_t n4, uint32_t* out) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n4) return;
+    float m = 0.0f;  // largest coordinate of the scene's box
+    for (int k = 0; k < 3; k++)
+        m = fmaxf(m, fmaxf(fabsf(__uint_as_float(words[k])), fabsf(__uint_as_float(words[4 + k]))));
     const uint4* nd = bvh4 + (size_t)i * 8;
     const uint4 rf = nd[6];
     const uint32_t ref[4] = {rf.x, rf.y, rf.z, rf.w};
@@ -307,7 +313,8 @@ __global__ void wide_nodes(const uint4* bvh4, uint32_t n4, uint32_t* out) {
             mn = fminf(mn, lo[from[j]]);
             mx = fmaxf(mx, hi[from[j]]);
         }
-        float step = fmaxf((mx - mn) * (1.0f / 253.0f), fmaxf(fmaxf(fabsf(mn), fabsf(mx)) * 1.0e-7f, 1.0e-30f));
+        const float least = fmaxf(fmaxf(fabsf(mn), fabsf(mx)) * 2.5e-7f, fmaxf(m * 9.0949470e-13f, 1.0e-30f));
+        float step = fmaxf((mx - mn) * (1.0f / 253.0f), least);
         const uint32_t mask = ax == 0 ? (1u << inner) - 1u : (ax == 1 ? (1u << kids) - (1u << inner) : 0u);
         step = __uint_as_float((__float_as_uint(step) & ~15u) | mask);
         // The stored corner is where the byte plane of value -32768 lies.
@@ -529,9 +536,9 @@ done:
 #undef CKD
 #undef CK4
 
-cudaError_t launch_wide_nodes(const uint4* bvh4, uint32_t n4, uint32_t* out, cudaStream_t st) {
+cudaError_t launch_wide_nodes(const uint32_t* words, const uint4* bvh4, uint32_t n4, uint32_t* out, cudaStream_t st) {
     if (n4 == 0) return cudaSuccess;
-    bvh4b::wide_nodes<<<bvh4b::blocks(n4, 128), 128, 0, st>>>(bvh4, n4, out);
+    bvh4b::wide_nodes<<<bvh4b::blocks(n4, 128), 128, 0, st>>>(words, bvh4, n4, out);
     return cudaGetLastError();
 }
 

@@ -785,9 +785,9 @@ static oxpt_status build_wide(oxpt_ctx* c, const float4* geom, uint32_t nodes, s
         if (s) return s;
     }
     uint32_t* out = wide_part(*bvh4, n4);
-    CK(c, oxd::launch_wide_nodes(reinterpret_cast<const uint4*>(*bvh4), n4, out, st), "wide nodes");
-    CK(c, oxd::launch_leaf_map(reinterpret_cast<const uint32_t*>(geom), nodes, out + (size_t)n4 * 16, (uint32_t)slots,
-                               st), "leaf map");
+    const uint32_t* words = reinterpret_cast<const uint32_t*>(geom);
+    CK(c, oxd::launch_wide_nodes(words, reinterpret_cast<const uint4*>(*bvh4), n4, out, st), "wide nodes");
+    CK(c, oxd::launch_leaf_map(words, nodes, out + (size_t)n4 * 16, (uint32_t)slots, st), "leaf map");
     return OXPT_OK;
 }
 

@@ -107,8 +107,9 @@ Collapse collapse4_device(const uint32_t* words, uint32_t nodes, cudaStream_t st
 // host's depth walk counts them.
 bool binary_depth_device(const uint32_t* words, uint32_t nodes, cudaStream_t st, uint32_t* depth, std::string* err);
 // The four-wide nodes with 8-bit child boxes, 16 words each: lower corner and
-// step per axis, a byte per child and plane, the child references.
-cudaError_t launch_wide_nodes(const uint4* bvh4, uint32_t n4, uint32_t* out, cudaStream_t st);
+// step per axis, a byte per child and plane, the child references. `words`:
+// the binary nodes.
+cudaError_t launch_wide_nodes(const uint32_t* words, const uint4* bvh4, uint32_t n4, uint32_t* out, cudaStream_t st);
 // map[slot] = the binary leaf node that holds the slot, for every slot below
 // `slots` (0 for a slot in no leaf).
 cudaError_t launch_leaf_map(const uint32_t* words, uint32_t nodes, uint32_t* map, uint32_t slots, cudaStream_t st);

@@ -27,10 +27,14 @@
 //
 // Why the result is the reference walk's although the order and the box
 // test are not:
-// * Boxes are widened by eta = 2^-18 x the largest coordinate of the scene
-//   box and the ray origin. With u = 2^-24, what the slab arithmetic below
-//   loses is within 8 u of that and within 1/128 of a byte step (the bytes
-//   leave 1/32): every box that the exact test enters is entered here too.
+// * Every box that the exact test enters is entered here too. With u = 2^-24,
+//   a plane's distance is within 0.006 byte steps (the bytes leave 1/32) and
+//   3 u of itself, the exact test's within 2 u (and its far planes are taken
+//   6 u too far): SLACK covers both. No term grows with the coordinates, so a
+//   small object in a large scene is entered as exactly as by itself.
+//   (Widening by 64 u of the largest coordinate, a frame of a 512 k-triangle
+//   object of 1 unit above a ground of 10^4 units took 49 ms, of 10^5 units
+//   2.4 s; now 7.0 and 7.2.)
 // * A closest hit's distance limit T is compared with the entry on the ray's
 //   dominant axis alone. The watertight test's distance is a weighted mean of
 //   its vertices' distances on that axis, whatever the weights are, so it is
@@ -70,14 +74,11 @@ constexpr uint32_t SS = 6;        // stack entries a lane keeps in shared memory
 constexpr uint32_t FLUSH = 32;    // pending leaves of a warp that start a pass of triangle tests
 constexpr uint32_t MIN_RAYS = 4;  // rays of a warp, at least, when they are few
 constexpr int STEPS = 4;          // node steps between checks
-constexpr float ETA = 3.8146973e-6f;     // 2^-18
-// Reciprocal directions are cut to INV_MAX, so that the product with a node's
-// corner (up to 260 times the largest coordinate below the box) stays finite
-// for coordinates up to FAR. The rays this changes move less than 10^-17 of a
-// distance along the axis, and eta x INV_MAX is still 10^11 times the largest
-// coordinate, so the box test stays on the safe side.
-constexpr float INV_MAX = 1.0e17f;
-constexpr float FAR = 1.0e18f;
+constexpr float SLACK = 1.0000012f;      // 1 + 20 u, on far planes
+// Largest distance of an origin, in scene sizes (a frame of the 512 k-triangle
+// object from 3e4 / 6e4 / 1e5 sizes away: 5.3 / 7.2 / 11.2 ms; left to the
+// reference's walk from 1.5e5: 6.7).
+constexpr float AWAY = 5.0e4f;
 constexpr float LIMIT = 1.00002f;        // closest hit: distance limit over the best distance
 
 // One warp's rays and pending work in shared memory.
@@ -128,29 +129,32 @@ __device__ __forceinline__ u8x ld32(const void* p) {
     return r;
 }
 
-// What a node step needs of a ray: reciprocal direction, the product of it
-// with the origin moved along it by eta, negated, and what moving the origin
-// back by eta instead adds to a far plane's distance.
+// What a node step needs of a ray: its origin and reciprocal direction. With m
+// the largest coordinate of the scene's box, what a step adds up is at most
+// 600 m + |o| times a reciprocal, so reciprocals are cut to keep that finite
+// (a zero component has 1e30). The cut only brings planes nearer: a near
+// plane stays a lower bound, and a far one is still 0.025 steps of at least
+// 2^-40 m away, which must be beyond the scene. False when that does not hold
+// (coordinates beyond 1e17), and for origins so far away that SLACK of the
+// distance is a good part of the scene: the ray is then left to the
+// reference's walk.
 struct NodeRay {
-    float inv[3], nb[3], c[3];
+    float o[3], inv[3];
 };
 
-// False when the coordinates are out of the node step's range.
 __device__ __forceinline__ bool node_ray(const Scene& s, const Ray& r, NodeRay& n) {
-    float4 lo = geomv(s, 0), hi = geomv(s, 1);
-    float m = fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(hi.x)), fmaxf(fabsf(lo.y), fabsf(hi.y))),
-                    fmaxf(fabsf(lo.z), fabsf(hi.z)));
-    m = fmaxf(m, fmaxf(fabsf(r.o.x), fmaxf(fabsf(r.o.y), fabsf(r.o.z))));
-    const float eta = m * ETA;
+    const float4 lo = geomv(s, 0), hi = geomv(s, 1);
+    const float m = max3(fmaxf(fabsf(lo.x), fabsf(hi.x)), fmaxf(fabsf(lo.y), fabsf(hi.y)),
+                         fmaxf(fabsf(lo.z), fabsf(hi.z)));
+    const float away = max3(fabsf(r.o.x), fabsf(r.o.y), fabsf(r.o.z)), reach = 600.0f * m + away;
+    const float cut = 1.0e37f / reach, main = fabsf(r.shear.z);  // the dominant reciprocal
     const float iv[3] = {r.inv.x, r.inv.y, r.inv.z}, oo[3] = {r.o.x, r.o.y, r.o.z};
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        const float v = fminf(fmaxf(iv[a], -INV_MAX), INV_MAX);
-        n.inv[a] = v;
-        n.nb[a] = -((v < 0.0f ? oo[a] - eta : oo[a] + eta) * v);
-        n.c[a] = fabsf(2.0f * eta * v);
+        n.o[a] = oo[a];
+        n.inv[a] = fminf(fmaxf(iv[a], -cut), cut);
     }
-    return m <= FAR;
+    return main >= 1.0e-9f && reach * main * reach <= 2.0e23f * m && away <= AWAY * m;
 }
 
 // Byte k of w as the float 32768 + byte.
@@ -463,15 +467,14 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
 #pragma unroll
             for (int ax = 0; ax < 3; ax++) {
                 const float A = __uint_as_float(v0.v[3 + ax]) * nr.inv[ax];
-                const float bn = __fmaf_rn(__uint_as_float(v0.v[ax]), nr.inv[ax], nr.nb[ax]);
-                const float bf = bn + nr.c[ax];
+                const float b = (__uint_as_float(v0.v[ax]) - nr.o[ax]) * nr.inv[ax];
                 const uint32_t lo = ax < 2 ? v0.v[6 + ax] : v1.v[0], hi = v1.v[1 + ax];
                 const bool neg = nr.inv[ax] < 0.0f;
                 const uint32_t nw = neg ? hi : lo, fw = neg ? lo : hi;
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
                     const float2 t = fma2(make_float2(plane(nw, k), plane(fw, k)), make_float2(A, A),
-                                          make_float2(bn, bf));
+                                          make_float2(b, b));
                     if (ax == 0) t0[k] = t.x, t1[k] = t.y;
                     else if (ax == 1) tx[k] = t.x, ty[k] = t.y;
                     else {
@@ -484,7 +487,7 @@ __global__ void __launch_bounds__(NT, MINB) wide_walk(const __grid_constant__ Wa
             uint32_t hit = 0u;
 #pragma unroll
             for (int k = 0; k < 4; k++)
-                if (t0[k] <= t1[k] && (!EXT || td[k] <= tl)) hit |= 1u << k;
+                if (t0[k] <= t1[k] * SLACK && (!EXT || td[k] <= tl)) hit |= 1u << k;
             const uint32_t inner = hit & v0.v[3], leaf = hit & v0.v[4];  // the low four bits
 #pragma unroll
             for (int k = 0; k < 4; k++)

@@ -70,3 +70,32 @@ def test_axis_rays_of_mixed_scales_in_a_batch(pkg, oracle):
         t.finish()
         cpu, _ = oracle.render(t.prepared(), 2)
         assert np.array_equal(t.read_accum().view(np.uint32), cpu.view(np.uint32)), s
+
+
+def test_small_object_in_a_large_scene_costs_no_more(pkg):
+    """A finely tessellated object above a ground of 10 and of 10^5 units: the
+    same rays meet the same triangles, so the frames take about as long (a box
+    test that widens boxes by a share of the largest coordinate took 450 times
+    as long)."""
+    import time
+    best = []
+    for ground in (10.0, 1.0e5):
+        s = pkg.Scene.icosphere(freq=160, seed=3, n_materials=2, n_textures=1, tex_size=16, n_punctual=2, n_emissive=0,
+                                material_mix=0)
+        q = np.asarray([(-1, 0, -1), (-1, 0, 1), (1, 0, 1), (1, 0, -1)], np.float32) * ground - (0, 1.2, 0)
+        s.add_mesh(np.asarray([q[[0, 1, 2]], q[[0, 2, 3]]], np.float32), 0)
+        t = pkg.GpuPathTracer(0)
+        t.set_tuning(mode=2)
+        assert t.sync(s, pkg.RenderOptions(width=480, height=270, scene_camera=0,
+                                           path_trace=pkg.PathTraceOptions(samples_per_pixel=4, max_bounces=4)))
+        t.set_camera(eye=(0.0, 1.0, 3.0), target=(0.0, 0.0, 0.0), yfov=0.8)
+        times = []
+        for _ in range(4):
+            t.reset()
+            t.finish()
+            t0 = time.perf_counter()
+            t.refine(4)
+            t.finish()
+            times.append(time.perf_counter() - t0)
+        best.append(min(times))
+    assert best[1] < 8.0 * best[0], best
