@@ -345,6 +345,24 @@ __global__ void leaf_map(const uint32_t* w, uint32_t nodes, uint32_t* map, uint3
     for (uint32_t k = 0; k < count; k++) map[first + k] = i;
 }
 
+// Sets *outside when a leaf's triangle has a vertex outside the leaf's box.
+// The triangles follow the nodes, 12 words each.
+__global__ void leaf_contents(const uint32_t* w, uint32_t nodes, uint64_t words, uint32_t* outside) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nodes) return;
+    const BN n = load(w, i);
+    const uint64_t end = ((uint64_t)n.first + n.count) * 12u + (uint64_t)nodes * 8u;
+    if (n.count == 0u || end > words) return;
+    const float4* tri = reinterpret_cast<const float4*>(w) + (uint64_t)nodes * 2u + (uint64_t)n.first * 3u;
+    bool in = true;
+    for (uint32_t k = 0; k < 3u * n.count; k++) {
+        const float4 v = tri[k];
+        in = in && v.x >= n.lo[0] && v.y >= n.lo[1] && v.z >= n.lo[2] && v.x <= n.hi[0] && v.y <= n.hi[1] &&
+             v.z <= n.hi[2];
+    }
+    if (!in) atomicOr(outside, 1u);
+}
+
 unsigned blocks(uint32_t n, unsigned t) { return (n + t - 1) / t; }
 
 }  // namespace bvh4b
@@ -539,6 +557,14 @@ done:
 cudaError_t launch_wide_nodes(const uint32_t* words, const uint4* bvh4, uint32_t n4, uint32_t* out, cudaStream_t st) {
     if (n4 == 0) return cudaSuccess;
     bvh4b::wide_nodes<<<bvh4b::blocks(n4, 128), 128, 0, st>>>(words, bvh4, n4, out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_leaf_contents(const uint32_t* words, uint32_t nodes, uint64_t count, uint32_t* outside,
+                                 cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(outside, 0, 4, st);
+    if (e != cudaSuccess || nodes == 0) return e;
+    bvh4b::leaf_contents<<<bvh4b::blocks(nodes, 256), 256, 0, st>>>(words, nodes, count, outside);
     return cudaGetLastError();
 }
 

@@ -45,7 +45,7 @@ struct SceneSet {
     uint32_t node_count = 0, bvh_depth = 0;
     float4* bvh4 = nullptr;
     size_t bvh4_cap = 0;
-    bool bvh4_built = false;
+    bool bvh4_built = false, bvh4_holds = false;
     uint32_t bvh4_nodes = 0, bvh4_root = 0xffffffffu, bvh4_need = 0;
     uint32_t* tables = nullptr;
     size_t table_words = 0, tables_cap = 0;
@@ -119,6 +119,7 @@ struct oxpt_ctx {
     // nodes what wide_walk.cu reads (wide_part below)
     float4* bvh4 = nullptr;
     bool bvh4_built = false;
+    bool bvh4_holds = false;  // every leaf's box holds the leaf's triangles
     uint32_t bvh4_nodes = 0, bvh4_root = 0xffffffffu, bvh4_need = 0;
     uint32_t shadow_walk = 0;
     uint32_t closest_walk = 0;  // 1: continuation rays on the four-wide tree (tolerance plan)
@@ -217,6 +218,12 @@ bool bvh4_usable(const oxpt_ctx* c) {
     return c->bvh4_built && c->params.env[3] == c->node_count && c->bvh_depth <= 64 && c->bvh4_need <= 64;
 }
 
+// The wide closest-hit walk needs what an uploaded tree may lack: triangles
+// inside their leaves' boxes (they were checked where the upload places them).
+bool wide_closest_usable(const oxpt_ctx* c) {
+    return bvh4_usable(c) && c->bvh4_holds && c->params.offs2[2] == 2u * c->node_count;
+}
+
 // Keeps an owned scene buffer that already holds `bytes` (and is at most
 // twice that) instead of freeing and allocating it again: a re-upload of the
 // same scene then costs only its copies.
@@ -286,6 +293,7 @@ void swap_scene(oxpt_ctx* c) {
     std::swap(c->bvh4, b.bvh4);
     std::swap(c->bvh4_cap, b.bvh4_cap);
     std::swap(c->bvh4_built, b.bvh4_built);
+    std::swap(c->bvh4_holds, b.bvh4_holds);
     std::swap(c->bvh4_nodes, b.bvh4_nodes);
     std::swap(c->bvh4_root, b.bvh4_root);
     std::swap(c->bvh4_need, b.bvh4_need);
@@ -473,6 +481,7 @@ oxpt_status run_wave(oxpt_ctx* c, const oxd::TraceArgs& ta, bool count, const ox
     wa.l2_max_window = c->l2_max_window;
     wa.closest4 = (c->closest_walk && c->trace_variant >= 3 && bvh4_usable(c)) ? 1u : 0u;
     wa.wide = bvh4_usable(c) ? 1u : 0u;
+    wa.wide_closest = wide_closest_usable(c) ? 1u : 0u;
     // Stack depth: 32 entries are exact when the BVH has at most 32 levels.
     int sd = c->stack ? (int)c->stack : (c->bvh_depth <= 32 ? 32 : 64);
     bool four = c->shadow_walk == 0 && bvh4_usable(c);
@@ -522,7 +531,7 @@ int enqueue_iteration(oxpt_ctx* c, const oxd::WaveArgs& wa, const oxd::WaveArgs&
         run(5, [&] { return oxd::launch_split_shade(wa, count, (int)c->shade_variant, c->sms, st); });
         run(6, [&] { return oxd::launch_split_nee(wa, count, (int)c->nee_variant, c->sms, st); });
     }
-    const int sde = (wa.closest4 || (wa.wide && !count && c->trace_variant >= 3)) ? sd4 : sd;
+    const int sde = (wa.closest4 || (wa.wide_closest && !count && c->trace_variant >= 3)) ? sd4 : sd;
     if (wa.ray_order & 1u) {
         run(10, [&] { return oxd::launch_order_ext(wa, c->sms, st); });
         oxd::WaveArgs wo = wa;
@@ -776,9 +785,10 @@ static oxpt_status upload_bvh4(oxpt_ctx* c, const uint32_t* node_words, uint32_t
 }
 
 // Fills the part of the four-wide tree's buffer that wide_walk.cu reads, from
-// the scene's two trees, on `st`.
-static oxpt_status build_wide(oxpt_ctx* c, const float4* geom, uint32_t nodes, size_t slots, float4** bvh4,
-                              size_t* cap, uint32_t n4, cudaStream_t st) {
+// the scene's two trees, on `st`. With `holds` (trees that the library did not
+// build itself) the leaves' contents are checked too, and waited for.
+static oxpt_status build_wide(oxpt_ctx* c, const float4* geom, size_t geom_vec4, uint32_t nodes, size_t slots,
+                              float4** bvh4, size_t* cap, uint32_t n4, cudaStream_t st, bool* holds) {
     if (*cap < tree_bytes(n4, slots)) {  // a root that is a leaf: no nodes were stored
         oxpt_status s = realloc_dev(c, bvh4, tree_bytes(n4, slots), "four-wide tree");
         *cap = s ? 0 : tree_bytes(n4, slots);
@@ -787,6 +797,13 @@ static oxpt_status build_wide(oxpt_ctx* c, const float4* geom, uint32_t nodes, s
     uint32_t* out = wide_part(*bvh4, n4);
     const uint32_t* words = reinterpret_cast<const uint32_t*>(geom);
     CK(c, oxd::launch_wide_nodes(words, reinterpret_cast<const uint4*>(*bvh4), n4, out, st), "wide nodes");
+    if (holds) {
+        uint32_t outside = 1u, *flag = out + (size_t)n4 * 16;  // where the leaf map follows
+        CK(c, oxd::launch_leaf_contents(words, nodes, (uint64_t)geom_vec4 * 4u, flag, st), "leaf contents");
+        CK(c, cudaMemcpyAsync(&outside, flag, 4, cudaMemcpyDeviceToHost, st), "leaf contents");
+        CK(c, cudaStreamSynchronize(st), "leaf contents");
+        *holds = outside == 0u;
+    }
     CK(c, oxd::launch_leaf_map(words, nodes, out + (size_t)n4 * 16, (uint32_t)slots, st), "leaf map");
     return OXPT_OK;
 }
@@ -794,8 +811,9 @@ static oxpt_status build_wide(oxpt_ctx* c, const float4* geom, uint32_t nodes, s
 // The four-wide tree of the scene now in c->geom, collapsed on the device
 // (the host collapse's words); a tree too wide or deep for the device pass
 // is read back and collapsed on the host.
-static oxpt_status device_bvh4(oxpt_ctx* c, oxd::Arena* mem = nullptr) {
+static oxpt_status device_bvh4(oxpt_ctx* c, bool own_tree, oxd::Arena* mem = nullptr) {
     c->bvh4_built = false;
+    c->bvh4_holds = own_tree;  // a build's boxes are made from the triangles
     uint32_t* out = reinterpret_cast<uint32_t*>(c->bvh4);  // reused when large enough
     uint32_t n4 = 0, root = 0xffffffffu, need = 1;
     std::string e;
@@ -816,8 +834,8 @@ static oxpt_status device_bvh4(oxpt_ctx* c, oxd::Arena* mem = nullptr) {
         c->bvh4_need = need;
     }
     c->bvh4_built = false;
-    if (oxpt_status s = build_wide(c, c->geom, c->node_count, c->slot_count, &c->bvh4, &c->bvh4_cap, c->bvh4_nodes,
-                                   c->stream))
+    if (oxpt_status s = build_wide(c, c->geom, c->geom_vec4, c->node_count, c->slot_count, &c->bvh4, &c->bvh4_cap,
+                                   c->bvh4_nodes, c->stream, own_tree ? nullptr : &c->bvh4_holds))
         return s;
     c->bvh4_built = true;
     return OXPT_OK;
@@ -861,7 +879,7 @@ oxpt_status oxpt_upload_scene(oxpt_ctx* c, const oxpt_scene_desc* d) {
         c->bvh_depth = depth;
     }
     if (c->stack == 32 && c->bvh_depth > 32) c->stack = 0;
-    if ((s = device_bvh4(c))) return s;
+    if ((s = device_bvh4(c, false))) return s;
     c->has_scene = true;
     return OXPT_OK;
 }
@@ -926,7 +944,9 @@ oxpt_status oxpt_stage_scene(oxpt_ctx* c, const oxpt_scene_desc* d, const uint32
         b.bvh4_nodes = n4;
         b.bvh4_root = root;
         b.bvh4_need = need;
-        if ((s = build_wide(c, b.geom, b.node_count, b.slot_count, &b.bvh4, &b.bvh4_cap, n4, c->upload))) return s;
+        if ((s = build_wide(c, b.geom, b.geom_vec4, b.node_count, b.slot_count, &b.bvh4, &b.bvh4_cap, n4, c->upload,
+                            &b.bvh4_holds)))
+            return s;
         b.bvh4_built = true;
     }
     // REFUSED / UNSUPPORTED: the binary walk serves every ray of this scene.
@@ -987,7 +1007,7 @@ oxpt_status oxpt_build_scene(oxpt_ctx* c, const oxpt_scene_src* src, uint32_t* l
     c->bvh_depth = std::min(ds.depth, 65u);  // bvh_depth_of's cap
     if (c->stack == 32 && c->bvh_depth > 32) c->stack = 0;
     c->build_mem.rewind(0);  // the build's pieces: it waited for its streams
-    s = device_bvh4(c, &c->build_mem);
+    s = device_bvh4(c, true, &c->build_mem);
     if (!s && c->build_mem.bytes() > oxd::Arena::KEEP)
         CK(c, cudaStreamSynchronize(c->stream), "scene build");  // the block goes back
     c->build_mem.end();
@@ -1066,6 +1086,7 @@ oxpt_status oxpt_share_scene(oxpt_ctx* c, const oxpt_ctx* owner) {
     c->bvh_depth = owner->bvh_depth;
     c->bvh4 = owner->bvh4;
     c->bvh4_built = owner->bvh4_built;
+    c->bvh4_holds = owner->bvh4_holds;
     c->bvh4_nodes = owner->bvh4_nodes;
     c->bvh4_root = owner->bvh4_root;
     c->bvh4_need = owner->bvh4_need;
@@ -1730,7 +1751,7 @@ oxpt_status batch_graph_run(oxpt_ctx* e, const std::vector<oxd::WaveArgs>& args,
         // node words (one-scene batches), the walk's storage split and tree.
         const oxd::WaveArgs& a0 = args[0];
         key.insert(key.end(), {(uint64_t)(uintptr_t)a0.s.geom, a0.s.geom_vec4, a0.s.P.env[3], a0.one_scene,
-                               a0.closest4, a0.wide, a0.walk_lim, a0.walk_stage, (uint64_t)(uintptr_t)a0.st.vis,
+                               a0.closest4, a0.wide, a0.wide_closest, a0.walk_lim, a0.walk_stage, (uint64_t)(uintptr_t)a0.st.vis,
                                a0.shadow_post, a0.ray_order, a0.l2_share, a0.l2_max_window, a0.one_frame});
         if (a0.one_frame) {
             // The scene in the kernels' arguments; the camera and the seed come
@@ -1977,9 +1998,12 @@ oxpt_status oxpt_refine_batch(oxpt_ctx* e, const oxpt_batch_frame* fr, uint32_t 
         wa.total = total;
         args.push_back(wa);
     }
-    bool wide = true;  // every frame's scene has its four-wide tree
-    for (uint32_t k = 0; k < n; k++)
-        if (fr[k].count && fr[k].rows && !bvh4_usable(fr[k].ctx)) wide = false;
+    bool wide = true, wide_closest = true;  // every frame's scene has its four-wide tree
+    for (uint32_t k = 0; k < n; k++) {
+        if (!fr[k].count || !fr[k].rows) continue;
+        wide = wide && bvh4_usable(fr[k].ctx);
+        wide_closest = wide_closest && wide_closest_usable(fr[k].ctx);
+    }
     const bool closest4 = e->closest_walk && e->trace_variant >= 3 && wide;
     oxd::WaveArgs base{};
     {
@@ -2021,6 +2045,7 @@ oxpt_status oxpt_refine_batch(oxpt_ctx* e, const oxpt_batch_frame* fr, uint32_t 
         wa.l2_max_window = e->l2_max_window;
         wa.closest4 = closest4 ? 1u : 0u;
         wa.wide = wide ? 1u : 0u;
+        wa.wide_closest = wide_closest ? 1u : 0u;
         wa.total = total;
         wa.out = e->out;
         wa.counters = nullptr;

@@ -113,6 +113,10 @@ cudaError_t launch_wide_nodes(const uint32_t* words, const uint4* bvh4, uint32_t
 // map[slot] = the binary leaf node that holds the slot, for every slot below
 // `slots` (0 for a slot in no leaf).
 cudaError_t launch_leaf_map(const uint32_t* words, uint32_t nodes, uint32_t* map, uint32_t slots, cudaStream_t st);
+// *outside = 1 when some leaf's triangle has a vertex outside the leaf's box,
+// else 0; `count`: words of the nodes and the triangles behind them.
+cudaError_t launch_leaf_contents(const uint32_t* words, uint32_t nodes, uint64_t count, uint32_t* outside,
+                                 cudaStream_t st);
 
 namespace prep {
 

@@ -152,9 +152,10 @@ struct WaveArgs {
     // continuation rays walk the four-wide tree (traversal variants 3-5;
     // the tolerance plan: closest hits equal except near-ties)
     uint32_t closest4 = 0u;
-    // every scene of the launch has its four-wide tree: the walks of
-    // variants 3-5 may use wide_walk.cu
-    uint32_t wide = 0u;
+    // every scene of the launch has its four-wide tree: the shadow walks of
+    // variants 3-5 may use wide_walk.cu; wide_closest: and its leaves hold
+    // their triangles, so that the closest-hit walks may too
+    uint32_t wide = 0u, wide_closest = 0u;
     // four-wide shadow walks of variants 3-5 park leaves until the warp
     // has no node work (same occlusion, fewer mixed node/leaf steps)
     uint32_t shadow_post = 0u;

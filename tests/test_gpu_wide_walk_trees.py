@@ -199,3 +199,9 @@ def _same(pkg, oracle, p, staged):
 def test_sliver_hit_before_its_box_begins(pkg, oracle, staged):
     s = _sliver()
     _same(pkg, oracle, _prepared(pkg, s, (s.min(0), s.max(0))), staged)
+
+
+@pytest.mark.parametrize("staged", [False, True])
+@pytest.mark.parametrize("hit", [1.0, 1.45])
+def test_triangle_outside_its_leafs_box(pkg, oracle, hit, staged):
+    _same(pkg, oracle, _prepared(pkg, _facing(hit), _box(1.8, 2.4, 0.05)), staged)
