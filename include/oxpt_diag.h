@@ -86,7 +86,9 @@ oxpt_status oxpt_diag_counters_split(const oxpt_ctx* ctx, uint64_t out[16]);
 oxpt_status oxpt_diag_set_launch(oxpt_ctx* ctx, uint32_t threads, uint32_t blocks_per_sm,
                                  uint64_t max_paths_per_launch);
 
-/* Traversal kernels of trace_variant 3-5: walk-stack entries per lane kept
+/* Short-stack traversal kernels of trace_variant 3-5 (those of counting
+ * runs, binary or postponed shadow walks, the tolerance plan and scenes that
+ * the wide walk does not serve): walk-stack entries per lane kept
  * in shared memory (at most 16; deeper entries live in local memory) and
  * the number of top nodes of the binary tree each CTA stages in shared
  * memory (within what the variant's occupancy leaves a block). Both only
@@ -100,10 +102,11 @@ oxpt_status oxpt_diag_get_walk(const oxpt_ctx* ctx, uint32_t out[2]);
  * are stored, 0 = a pending record per job with a visibility word. The
  * logic kernel adds the same contributions in the same order either way. */
 oxpt_status oxpt_diag_set_nee_mask(oxpt_ctx* ctx, int on);
-/* Four-wide shadow walks of trace_variant 3-5: 1 = lanes park the leaves
+/* Shadow walks of trace_variant 3-5 on the four-wide tree: 1 = short-stack
+ * kernels whose lanes park the leaves
  * they reach and keep walking inner nodes, and the warp tests parked
  * leaves together once no lane has node work left (speculative traversal);
- * 0 (default) = each lane tests a leaf when it reaches it. Occlusion does
+ * 0 (default) = the wide walk. Occlusion does
  * not depend on the order, so results are the same. */
 oxpt_status oxpt_diag_set_shadow_postpone(oxpt_ctx* ctx, int on);
 /* Wavefront plans, bit 0: before the closest-hit walk the continuation
@@ -114,9 +117,9 @@ oxpt_status oxpt_diag_set_shadow_postpone(oxpt_ctx* ctx, int on);
  * walked alone by one lane, so results are the same either way. The
  * reordering launches time as kind 10. */
 oxpt_status oxpt_diag_set_ray_order(oxpt_ctx* ctx, int mode);
-/* on = 1: the short-stack traversal kernels (trace_variant 3-5) of launches
- * over one scene mark the tree nodes they read (the binary nodes for
- * closest hits, the four-wide tree for shadow rays) as persisting L2 lines
+/* on = 1: the traversal kernels of trace_variant 3-5, in launches over one
+ * scene, mark the tree nodes they read (the wide nodes, or the short-stack
+ * kernels' binary or four-wide nodes) as persisting L2 lines
  * through an access-policy window, half of the L2 set-aside each; the
  * process's persisting set-aside is raised to the device maximum, a limit
  * of this process's CUDA context. *granted (optional) = the set-aside in

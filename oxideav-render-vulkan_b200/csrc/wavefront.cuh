@@ -191,6 +191,23 @@ cudaError_t launch_wave_shadow(const WaveArgs& a, bool count, bool four, int var
 // (four: the four-wide tree); variant 0..2 targets 6 / 8 / 10 blocks per SM.
 cudaError_t launch_walk(const WaveArgs& a, bool count, bool ext, bool four, int variant, int sd, int sms,
                         cudaStream_t st);
+// The launch attribute that marks the tree nodes a walk reads as persisting L2
+// lines, so that the wavefront state and attributes streaming through L2
+// between walks do not evict them (a hint: results do not depend on it).
+// Returns the number of attributes set: 0 when the option is off or the launch
+// traces several scenes.
+inline unsigned l2_window(const WaveArgs& a, const void* base, uint64_t bytes, cudaLaunchAttribute* attr) {
+    if (!a.l2_share || !a.l2_max_window || !base || !bytes || (a.nframes != 0 && !a.one_scene)) return 0u;
+    const uint64_t win = bytes < a.l2_max_window ? bytes : a.l2_max_window;
+    const double ratio = (double)a.l2_share / (double)win;
+    attr->id = cudaLaunchAttributeAccessPolicyWindow;
+    attr->val.accessPolicyWindow.base_ptr = const_cast<void*>(base);
+    attr->val.accessPolicyWindow.num_bytes = (size_t)win;
+    attr->val.accessPolicyWindow.hitRatio = ratio < 1.0 ? (float)ratio : 1.0f;
+    attr->val.accessPolicyWindow.hitProp = cudaAccessPropertyPersisting;
+    attr->val.accessPolicyWindow.missProp = cudaAccessPropertyNormal;
+    return 1u;
+}
 // wide_walk.cu: closest hits (ext) or shadow rays over the four-wide tree with
 // the reference walk's results; sd: stack entries (32 or 64, the tree's need).
 cudaError_t launch_wide_walk(const WaveArgs& a, bool ext, int variant, int sd, int sms, cudaStream_t st);

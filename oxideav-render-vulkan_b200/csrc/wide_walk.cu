@@ -592,7 +592,14 @@ cudaError_t launch_wide_walk(const WaveArgs& a, bool ext, int variant, int sd, i
     if (e != cudaSuccess) return e;
     WaveArgs copy = a;
     void* args[] = {&copy};
-    return cudaLaunchKernel(fn, dim3((unsigned)(sms * (per_sm > 0 ? per_sm : 1))), dim3(NT), args, 0, st);
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sms * (per_sm > 0 ? per_sm : 1)));
+    cfg.blockDim = dim3(NT);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = l2_window(a, a.s.wide, (uint64_t)a.s.bvh4_nodes * 64u, attr);
+    return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
 }  // namespace oxd
