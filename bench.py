@@ -527,9 +527,10 @@ def run_walk_sweep(a):
     """Traversal-kernel sweep on the single large scene: per-launch CUDA-event
     times of the extension and shadow kernels, summed over a `--spp` refine
     of the frame (graphs off, so every launch is timed), for each traversal
-    variant (0-2 local-memory stacks at 6 / 8 / 10 blocks per SM; 3-5
-    shared-memory short stacks at 6 / 8 / 10), stack entries kept on chip and
-    staged top nodes, and the tolerance plan. One JSON line per point."""
+    variant (0-2 local-memory stacks at 6 / 8 / 10 blocks per SM; 3 and 4 the
+    wide walk at 6 / 8), the short-stack kernels of 3-5 (binary shadow rays)
+    by stack entries kept on chip and staged top nodes, and the tolerance
+    plan. One JSON line per point."""
     import torch
     torch.cuda.set_device(0)
     __graft_entry__.build()
@@ -547,8 +548,8 @@ def run_walk_sweep(a):
     spp = min(a.spp, 8)
     line_extra = {}
 
-    def run(tv, lim, stage, closest=0):
-        t.set_tuning(trace_variant=tv, closest_walk=closest)
+    def run(tv, lim, stage, closest=0, shadow=0):
+        t.set_tuning(trace_variant=tv, closest_walk=closest, shadow_walk=shadow)
         L.oxpt_diag_set_walk(ctx, lim, stage)
         t.reset()
         t.refine(spp)
@@ -564,17 +565,17 @@ def run_walk_sweep(a):
         L.oxpt_diag_timing_kinds(ctx, kms, kn)
         line = {"workload": f"traversal sweep, single large scene 1920x1080, {spp} spp, graphs off",
                 "trace_variant": tv, "stack_entries_on_chip": lim, "staged_nodes": stage, "closest_walk": closest,
-                "extend_ms": kms[3], "shadow_ms": kms[4], "order_ms": kms[10],
+                "shadow_walk": shadow, "extend_ms": kms[3], "shadow_ms": kms[4], "order_ms": kms[10],
                 "frame_kernels_ms": sum(kms[k] for k in (2, 3, 4, 5, 6, 10))}
         line.update(line_extra)
         print(json.dumps(line), flush=True)
 
-    for tv in (0, 1, 2):
+    for tv in (0, 1, 2, 3, 4):
         run(tv, 2, 0)
     for tv in (3, 4, 5):
         for lim in (0, 2, 4, 8, 16):
             for stage in (0, 127, 511):
-                run(tv, lim, stage)
+                run(tv, lim, stage, shadow=1)
     for tv in (3, 4):
         for lim in (2, 8):
             run(tv, lim, 0, closest=1)
