@@ -490,6 +490,7 @@ done:
         if (p && !mem) cudaFreeAsync(p, st);
     if (res != Collapse::BUILT) {
         cudaStreamSynchronize(st);
+        (void)cudaGetLastError();  // a failed allocation is the caller's to report
         *n4 = 0;
     }
     return res;

@@ -971,6 +971,13 @@ oxpt_status oxpt_build_scene(oxpt_ctx* c, const oxpt_scene_src* src, uint32_t* l
     auto t0 = std::chrono::steady_clock::now();
     oxd::prep::DeviceScene ds;
     std::string e;
+    auto free_scene = [c] {
+        realloc_dev(c, &c->geom, 0, "geom buffer");
+        realloc_dev(c, &c->attrs, 0, "attribute buffer");
+        realloc_dev(c, &c->atlas, 0, "texture atlas");
+        realloc_dev(c, &c->bvh4, 0, "four-wide tree");
+        c->geom_cap = c->attrs_cap = c->atlas_cap = c->bvh4_cap = 0;
+    };
     for (int attempt = 0;; attempt++) {
         ds.geom = c->geom;
         ds.geom_cap = c->geom_cap;
@@ -987,14 +994,11 @@ oxpt_status oxpt_build_scene(oxpt_ctx* c, const oxpt_scene_src* src, uint32_t* l
         c->atlas_cap = ds.atlas_cap;
         if (s != OXPT_E_NOMEM || attempt) break;
         // Short of memory: the old scene's buffers go first.
-        realloc_dev(c, &c->geom, 0, "geom buffer");
-        realloc_dev(c, &c->attrs, 0, "attribute buffer");
-        realloc_dev(c, &c->atlas, 0, "texture atlas");
-        realloc_dev(c, &c->bvh4, 0, "four-wide tree");
-        c->geom_cap = c->attrs_cap = c->atlas_cap = c->bvh4_cap = 0;
-        c->build_mem.end();
+        free_scene();
+        c->build_mem.drop();
     }
     if (s) {
+        free_scene();  // no scene is left, so nothing holds memory for one
         c->build_mem.end();
         return fail(c, s, e);
     }
@@ -1006,8 +1010,13 @@ oxpt_status oxpt_build_scene(oxpt_ctx* c, const oxpt_scene_src* src, uint32_t* l
     c->node_count = ds.node_count;
     c->bvh_depth = std::min(ds.depth, 65u);  // bvh_depth_of's cap
     if (c->stack == 32 && c->bvh_depth > 32) c->stack = 0;
-    c->build_mem.rewind(0);  // the build's pieces: it waited for its streams
+    c->build_mem.rewind();  // the build's pieces: it waited for its streams
     s = device_bvh4(c, true, &c->build_mem);
+    if (s) {  // the scratch block may have been in the way
+        c->build_mem.drop();
+        s = device_bvh4(c, true);
+        if (s) free_scene();
+    }
     if (!s && c->build_mem.bytes() > oxd::Arena::KEEP)
         CK(c, cudaStreamSynchronize(c->stream), "scene build");  // the block goes back
     c->build_mem.end();

@@ -46,10 +46,8 @@ class Arena {
         if (e == cudaSuccess) more_.push_back(own);
         return e;
     }
-    // Pieces handed out since `mark` are free again (a caller's piece
-    // outside the block stays until release).
-    size_t mark() const { return used_; }
-    void rewind(size_t mark) { used_ = mark; }
+    // The block's pieces are free again (pieces outside it stay until release).
+    void rewind() { used_ = 0; }
     void release() {
         used_ = 0;
         for (void* p : more_) cudaFree(p);
@@ -60,18 +58,18 @@ class Arena {
         release();
         if (cap_ > KEEP) drop();
     }
-    size_t bytes() const { return cap_; }
-    Arena() = default;
-    Arena(const Arena&) = delete;
-    Arena& operator=(const Arena&) = delete;
-
-  private:
     void drop() {
         release();
         if (base_) cudaFree(base_);
         base_ = nullptr;
         cap_ = 0;
     }
+    size_t bytes() const { return cap_; }
+    Arena() = default;
+    Arena(const Arena&) = delete;
+    Arena& operator=(const Arena&) = delete;
+
+  private:
     char* base_ = nullptr;
     size_t cap_ = 0, used_ = 0;
     std::vector<void*> more_;
