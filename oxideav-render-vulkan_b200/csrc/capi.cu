@@ -574,7 +574,7 @@ oxpt_status wave_loop(oxpt_ctx* c, const oxd::WaveArgs& wa, bool count, bool fou
     // iteration b + 3, whose path logic alone is left to run: nothing has to
     // be read back then (256 x 256, 8 bounces: 11 instead of 12 iterations and
     // two instead of three waits).
-    const uint64_t last = wa.total <= wa.slots ? std::min<uint64_t>(max_bounces, 1u << 20) + 3 : ~0ull;
+    const uint64_t last = wa.total <= wa.slots ? (uint64_t)max_bounces + 3 : ~0ull;
     for (uint64_t it = 0;; it++) {
         if (it > cap) return fail(c, OXPT_E_TIMEOUT, "wavefront did not drain within its iteration bound");
         cudaError_t e = cudaSuccess;
