@@ -152,8 +152,9 @@ oxpt_status oxpt_diag_set_l2_window(oxpt_ctx* ctx, int on, uint64_t* granted);
  *                  tree, with short stacks in shared memory, alpha tests
  *                  out of line and optional staged top nodes
  *                  (oxpt_diag_set_walk) for 6 / 8 / 10 blocks. Default 4.
- *   nee_variant    NEE kernel, punctual lights job-major (0, 1, 2) or
- *                  vertex-major (3, 4, 5) for 4 / 5 / 6 blocks.
+ *   nee_variant    NEE kernel, punctual lights job-major for 2 (0, 1) or 3
+ *                  (2) resident blocks of 256 threads per SM, or vertex-major
+ *                  for 2 (3, 4) or 3 (5).
  *   stack          traversal stack entries: 32 or 64; 0 = 32 when the BVH
  *                  is at most 32 levels deep, else 64 (exact either way).
  *   shadow_walk    wavefront shadow rays: 0 = the four-wide tree built on

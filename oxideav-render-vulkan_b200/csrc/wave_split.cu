@@ -529,7 +529,7 @@ __device__ __forceinline__ void put_job(const WaveArgs& a, uint32_t slot, uint32
 // warp evaluate the same light) or job-major (one thread per vertex and
 // light: batches that mix scenes of different light counts).
 template <bool VMAJOR, int MINB, int M>
-__global__ void __launch_bounds__(NEE_THREADS, MINB * 128 / NEE_THREADS) split_nee(const __grid_constant__ WaveArgs a) {
+__global__ void __launch_bounds__(NEE_THREADS, MINB) split_nee(const __grid_constant__ WaveArgs a) {
     constexpr bool BATCH = M == FRAMES;
     __shared__ float s_sheen[512];
     // Punctual lights of a one-scene launch, four 16-byte words each.
@@ -608,20 +608,16 @@ __global__ void __launch_bounds__(NEE_THREADS, MINB * 128 / NEE_THREADS) split_n
 
 // Variants: shade kernel for 2 (0, 1; 128 registers) or 3 (2; 80) blocks per
 // SM, 3.37 against 3.26 ms of shading per 8 spp of the 1.05 M-triangle frame,
-// 3.34 against 3.71 of 480 k-triangle boxes; the NEE kernel job-major (0-2) or
-// vertex-major (3-5) for 4 / 5 / 6 blocks of 128.
+// 3.34 against 3.71 of 480 k-triangle boxes; the NEE kernel job-major for 2
+// (0, 1) or 3 (2) blocks per SM, or vertex-major for 2 (3, 4) or 3 (5).
 template <bool C, int M>
 static void* shade_fn(int v) {
     return v < 2 ? (void*)split_shade<C, 2, M> : (void*)split_shade<C, 3, M>;
 }
 template <int M>
 static void* nee_fn(int v) {
-    if (v == 0) return (void*)split_nee<false, 4, M>;
-    if (v == 1) return (void*)split_nee<false, 5, M>;
-    if (v == 2) return (void*)split_nee<false, 6, M>;
-    if (v == 3) return (void*)split_nee<true, 4, M>;
-    if (v == 4) return (void*)split_nee<true, 5, M>;
-    return (void*)split_nee<true, 6, M>;
+    if (v < 3) return v < 2 ? (void*)split_nee<false, 2, M> : (void*)split_nee<false, 3, M>;
+    return v < 5 ? (void*)split_nee<true, 2, M> : (void*)split_nee<true, 3, M>;
 }
 
 // One grid of resident blocks, no more than the slots fill.

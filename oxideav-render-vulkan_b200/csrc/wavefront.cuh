@@ -36,7 +36,7 @@ struct WaveState {
     uint32_t* nee_n;           // NEE jobs of the last vertex to add (0..J)
     float4* pend;              // slots x J: contribution.xyz, 0 none / 1 queued / 2 visible
     uint32_t* frame;           // batched launches: the slot's frame
-    // split plan with at most 32 NEE jobs (else null): per slot, bit j set
+    // plans with at most 32 NEE jobs (else null): per slot, bit j set
     // when job j's shadow ray found nothing in the way; pend then holds
     // only the queued jobs' contributions and its w is not used
     uint32_t* vis;
@@ -99,7 +99,7 @@ struct WaveQueues {
     float4* sh_o;   // shadow ray origin, t_max
     float4* sh_d;   // shadow ray direction, skip id bits
     uint4* sh_m;    // slot, job, ray id, path seed
-    // split wavefront (wave_split.cu)
+    // shading (wave_split.cu)
     uint32_t* shade;  // slot ids with a surface hit to shade
     uint32_t* vslot;  // vertex record -> slot
     uint32_t* vlight;  // vertex records whose last NEE job samples the environment (from the
@@ -178,7 +178,7 @@ cudaError_t launch_order_shadow(const WaveArgs& a, int sms, cudaStream_t st);
 
 // Traversal. `variant`: 0..2, the occupancy target of the compiled kernel (6 /
 // 8 / 10 blocks per SM); 3..5 run wide_walk.cu, or wave_walk.cu for counting
-// launches, the binary shadow walk and scenes without a four-wide tree;
+// launches, the binary shadow walk and scenes that it does not serve;
 // `stack`: 32 or 64 entries.
 // With a.nframes > 0 the batched kernels run (count must then be false).
 cudaError_t launch_wave_extend(const WaveArgs& a, bool count, int variant, int stack, int sms, cudaStream_t st);
@@ -217,8 +217,8 @@ cudaError_t launch_wide_walk(const WaveArgs& a, bool ext, int variant, int sd, i
 // (the iteration's launches, this one included), tally[1] += 1.
 cudaError_t launch_wave_continue(cudaGraphConditionalHandle h, uint32_t* ctr, uint32_t cap, uint32_t* err,
                                  unsigned long long* tally, uint32_t kernels, cudaStream_t st);
-// Split wavefront (wave_split.cu); shade variants 2 / 3 / 4 blocks per SM,
-// NEE variants 4 / 5 / 6.
+// Shading (wave_split.cu). Shade variants: 2 (0, 1) or 3 (2) blocks per SM;
+// NEE variants: 2 (0, 1; 3, 4) or 3 (2; 5), job-major below 3.
 cudaError_t launch_split_logic(const WaveArgs& a, bool count, cudaStream_t st);
 cudaError_t launch_split_shade(const WaveArgs& a, bool count, int variant, int sms, cudaStream_t st);
 cudaError_t launch_split_nee(const WaveArgs& a, bool count, int variant, int sms, cudaStream_t st);
