@@ -1,10 +1,12 @@
 """Autotuner for the tracer's execution plan.
 
 Chooses, per scene and resolution, between the megakernel and the
-wavefront, and within the wavefront the shading kernel's register budget
-(shade_variant), the traversal kernels' occupancy target (trace_variant),
-the traversal stack depth, the number of paths in flight (wave_slots) and
-the shadow rays' tree (the four-wide any-hit tree or the binary walk).
+wavefront, and within the wavefront the surface shading kernel's register
+budget (shade_variant), the NEE kernel's and its order of punctual lights
+(nee_variant), the traversal kernels and their occupancy target
+(trace_variant), the traversal stack depth, the number of paths in flight
+(wave_slots) and the shadow rays' tree (the four-wide any-hit tree or the
+binary walk).
 Every plan yields bit-identical accumulators, so the tuner only measures
 time: each candidate runs a short refine at sample indices far from any
 real render's, timed with CUDA events on the tracer's stream, and the
@@ -44,13 +46,15 @@ class Plan:
                 self.shadow_walk, self.graphs, self.refill, self.closest_walk, self.fast_shading)
 
 
+# One value of each pair of variants that are the same kernels: shade_variant
+# 0 and 1, trace_variant 4 and 5, nee_variant 0 and 1, 3 and 4.
 SPACE = {
     "mode": [N.MODE_WAVEFRONT, N.MODE_WAVEFRONT_SPLIT, N.MODE_MEGAKERNEL],
-    "shade_variant": [0, 1, 2],
-    "trace_variant": [0, 1, 2, 3, 4, 5],
+    "shade_variant": [1, 2],
+    "trace_variant": [0, 1, 2, 3, 4],
     "stack": [0, 64],
     "wave_slots": [1 << 19, 1 << 20, 1 << 21, 1 << 22],
-    "nee_variant": [0, 1, 2, 3, 4, 5],
+    "nee_variant": [0, 2, 3, 5],
     "shadow_walk": [0, 1],
     "refill": [1, 8, 16, 32],
     "graphs": [0, 1],
@@ -65,7 +69,6 @@ LARGE_SCENE_WAVE_ITEMS = 1 << 27  # paths per launch round: a whole frame
 
 WAVE_ONLY = ("shade_variant", "trace_variant", "stack", "wave_slots", "nee_variant", "shadow_walk", "graphs",
              "refill")
-SPLIT_ONLY = ("nee_variant",)
 
 
 def coordinate_descent(measure: Callable[[Plan], float], start: Optional[Plan] = None,
@@ -85,8 +88,6 @@ def coordinate_descent(measure: Callable[[Plan], float], start: Optional[Plan] =
     best_cost = cost(best)
     for knob, values in space.items():
         if knob in WAVE_ONLY and best.mode == N.MODE_MEGAKERNEL:
-            continue
-        if knob in SPLIT_ONLY and best.mode != N.MODE_WAVEFRONT_SPLIT:
             continue
         for v in values:
             if getattr(best, knob) == v:
@@ -141,7 +142,7 @@ def tune_batch(tracers, executor, spp: int = 1, log: Optional[list] = None,
     synced): each candidate traces `spp` samples of every tracer at the
     tuner's sample indices as one batch, timed with CUDA events on the
     executor's stream; the tracers' accumulations are reset afterwards.
-    The megakernel is not a batch plan."""
+    The megakernel is not a batch plan, and the two wavefront modes are one."""
     L = N.lib()
     ctx = executor.ctx
     frames = (N.BatchFrame * len(tracers))()
@@ -150,7 +151,6 @@ def tune_batch(tracers, executor, spp: int = 1, log: Optional[list] = None,
         w, h = t.size()
         frames[k] = N.BatchFrame(t.ctx, TUNE_FIRST_SAMPLE, spp, 0, h)
     space = space or {k: v for k, v in SPACE.items() if k != "mode"}
-    space = {"mode": [N.MODE_WAVEFRONT_SPLIT, N.MODE_WAVEFRONT], **space}
 
     def measure(p: Plan) -> float:
         apply(executor, p)
