@@ -18,8 +18,8 @@
 // * A node step is about 190 instructions: the stored corner lets one fused
 //   operation place a plane, an any-hit walk takes its next node straight from
 //   the group of waiting siblings (nearest first gained it nothing).
-// A 64-spp 1080p frame of that scene: closest hits 89.9 -> 41 ms, shadow rays
-// 135.9 -> 67 ms (24 active lanes in a node step; now bound by issue: about 77%
+// A 64-spp 1080p frame of that scene: closest hits 89.9 -> 44 ms, shadow rays
+// 135.9 -> 70 ms (18 and 22 of 32 lanes active; now bound by issue: 71 and 73%
 // of cycles issue). FLUSH of 24 to 48, 4 to 10 entries in shared
 // memory, 2 to 8 steps between checks and 12 pending leaves were within 3%
 // of each other or worse; 48 registers a thread (10 blocks) spilled and were
